@@ -273,18 +273,30 @@ __global__ void __launch_bounds__(256) scatter_kernel(
 // skipping its own body (itself included); per-cell partial sums added to the total (the order
 // of FindAndHandleRigidBodyCollisionsUniformGridKernel, RigidBodies/UniformGridDEM.cu:166-193).
 // The particle's cell comes from its sorted key and its scene from the sorted velocity's w.
-// The three cells of an x-row are walked as one flattened loop (candidate t of the row maps to
-// cell a, b or c and to that cell's partial sum), so a warp's lanes stay in step across cells;
-// cells that hold only this particle's body are skipped from their tag without loading their
-// occupants, which could only be rejected.  Candidates at squared distance >= the float just
-// above (2r)^2 are rejected without the square root: for them sqrtf(d2) >= 2r exactly, so the
-// contact test is unchanged.
-struct RowCells {
-  uint2 a, b, c;
-};
+// The occupants of an x-row's cells are one run of the sorted slots, walked without telling the
+// cells apart; a contact, which is rare, finds its cell from its sorted key.  Cells that hold only
+// this particle's body are skipped from their tag without loading their occupants, which could
+// only be rejected.  Candidates at squared distance >= the float just above (2r)^2 are rejected
+// without the square root: for them sqrtf(d2) >= 2r exactly, so the contact test is unchanged.
+// Bound by issued instructions where cells are crowded (scenes folded into small grids; 2.1M
+// particles in 40 scenes: 227 -> 190 us against a walk that told the three cells apart and held
+// their partial sums) and by the latency of the 27 meta loads where they are not (2M pile: 58
+// us); loading 2, 4 or 8 candidates ahead changed nothing or lost occupancy.  Five blocks of 256
+// fit an SM with the scene table (a batch of one keeps its scene in the constant bank and more of
+// the rest in registers, where a fifth block spills and costs 2 %).
+// The meta word of a cell that holds only this body, count bits cleared (an impossible word when
+// the body has no tag).
+__device__ __forceinline__ uint32_t own_meta(uint32_t epoch, uint32_t btag) {
+  return btag ? (epoch << kEpochShift) | (btag << kTagShift) : 0xffffffffu;
+}
+// 1 for a cell with occupants to visit: not empty (another step's entry) and not only this body's.
+__device__ __forceinline__ uint32_t live_meta(uint32_t m, uint32_t epoch, uint32_t own) {
+  m &= ~kCountMask;
+  return ((m >> kEpochShift) & kEpochMask) == epoch && m != own ? 1u : 0u;
+}
 
 template <bool kOne>
-__global__ void __launch_bounds__(256, 4) collide_kernel(
+__global__ void __launch_bounds__(256, kOne ? 4 : 5) collide_kernel(
     const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table, int nt, const uint32_t* __restrict__ skeys,
     const uint32_t* __restrict__ svals, const uint2* __restrict__ cells,
     const float4* __restrict__ spos, const float4* __restrict__ svel,
@@ -298,13 +310,9 @@ __global__ void __launch_bounds__(256, 4) collide_kernel(
   const SceneDev& S = scene_at<kOne>(one, table, kOne ? 0 : __float_as_int(v4.w));
   const float3 pos = ar::xyz(p4), vel = ar::xyz(v4);
   const int body = __float_as_int(p4.w);
-  // the meta word of a cell holding only this body, count bits cleared (an impossible word
-  // when the body has no tag)
-  const uint32_t btag = body_tag(body - S.boff);
-  const uint32_t own = btag ? (epoch << kEpochShift) | (btag << kTagShift) : 0xffffffffu;
+  const uint32_t own = own_meta(epoch, body_tag(body - S.boff));
   const float thr = 2.0f * S.r;
   const float thr2_up = nextafterf(thr * thr, INFINITY);
-  const float kk = S.k, dmp = S.damping, shr = S.shear, att = S.attraction;
   const uint32_t lx = S.lx, ly = S.ly, mx = S.gx - 1, my = S.gy - 1, mz = S.gz - 1;
   const uint32_t base = S.cell_base, local = __ldg(skeys + k) - base;
   const uint32_t x = local & mx, y = (local >> lx) & my, z = local >> (lx + ly);
@@ -313,12 +321,7 @@ __global__ void __launch_bounds__(256, 4) collide_kernel(
     const uint32_t zz = (z + (uint32_t)(r / 3) - 1u) & mz, yy = (y + (uint32_t)(r % 3) - 1u) & my;
     return base + (zz << (lx + ly)) + (yy << lx);
   };
-  // a cell has occupants to visit unless it is empty (another step's entry) or holds only this
-  // particle's body
-  auto live = [&](uint32_t m) {
-    m &= ~kCountMask;
-    return ((m >> kEpochShift) & kEpochMask) == epoch && m != own ? 1u : 0u;
-  };
+  auto live = [&](uint32_t m) { return live_meta(m, epoch, own); };
   // pass 1: the meta words of all 27 cells (independent loads, all in flight together) ->
   // bit 3 r + i set when cell i (x-1, x, x+1) of row r has occupants to visit
   const uint32_t* __restrict__ meta = reinterpret_cast<const uint32_t*>(cells) + 1;
@@ -330,45 +333,51 @@ __global__ void __launch_bounds__(256, 4) collide_kernel(
                    mc = __ldg(meta + 2 * (rb + xc));
     todo |= (live(ma) | (live(mb) << 1) | (live(mc) << 2)) << (3 * r);
   }
-  // pass 2: rows with occupants to visit, in order.  A row without any would add +0 to every
-  // component of the total, which leaves it unchanged (the total starts at +0, and a float sum
-  // is -0 only when both addends are), so such rows are skipped.
-  auto visits = [&](const uint2& c, uint32_t cell) {  // a saturated count is resolved from the keys
-    if (!live(c.y)) return 0u;
-    uint32_t n = c.y & kCountMask;
-    if (n == kCountMask)
-      while (c.x + n < (uint32_t)nt && __ldg(skeys + c.x + n) == cell) ++n;
-    return n;
-  };
-  float3 lin = ar::mk3(0.f, 0.f, 0.f);
+  // pass 2: the cells with occupants to visit, in order, a segment of one row at a time.  A row
+  // that does not wrap has consecutive keys, so the occupants of its cells, from the first to
+  // the last one to visit, are one run of the sorted slots (a cell between them that holds only
+  // this body is walked through: its occupants are rejected); a row that wraps is taken a cell
+  // at a time.  A contact is added to its cell's partial sum, which joins the total when the
+  // cell changes: cells without contacts would add +0, which leaves the total unchanged (it
+  // starts at +0, and a float sum is -0 only when both addends are).
+  const bool wraps = x == 0 || x == mx;
+  float3 lin = ar::mk3(0.f, 0.f, 0.f), cf = lin;
   while (todo) {
     const int r = (__ffs(todo) - 1) / 3;
-    todo &= ~(7u << (3 * r));
+    uint32_t bits = (todo >> (3 * r)) & 7u;
+    if (wraps) bits &= 0u - bits;
+    todo &= ~(bits << (3 * r));
     const uint32_t row = row_base(r);
-    const RowCells cur{__ldg(cells + row + xa), __ldg(cells + row + x), __ldg(cells + row + xc)};
-    const uint32_t na = visits(cur.a, row + xa), nb = visits(cur.b, row + x),
-                   nc = visits(cur.c, row + xc);
-    const uint32_t nab = na + nb, total = nab + nc;
-    float3 fa = ar::mk3(0.f, 0.f, 0.f), fb = fa, fc = fa;
-    for (uint32_t t = 0; t < total; ++t) {
-      const uint32_t j = t < na ? cur.a.x + t : (t < nab ? cur.b.x + (t - na) : cur.c.x + (t - nab));
+    const uint32_t lo = row + ((x + (uint32_t)(__ffs(bits) - 2)) & mx);
+    const uint32_t hi = row + ((x + (uint32_t)(30 - __clz(bits))) & mx);
+    const uint2 last = __ldg(cells + hi);
+    uint32_t j = lo == hi ? last.x : __ldg(cells + lo).x;
+    uint32_t n = last.y & kCountMask;
+    if (n == kCountMask)  // a saturated count is resolved from the keys
+      while (last.x + n < (uint32_t)nt && __ldg(skeys + last.x + n) == hi) ++n;
+    const uint32_t end = last.x + n;
+    lin = ar::add(lin, cf);
+    cf = ar::mk3(0.f, 0.f, 0.f);
+    uint32_t cell = 0xffffffffu;
+    for (; j < end; ++j) {
       const float4 q4 = __ldg(spos + j);
-      if (__float_as_int(q4.w) == body) continue;
       const float3 rp = ar::sub(ar::xyz(q4), pos);
       const float d2 = ar::dot(rp, rp);
-      if (!(d2 < thr2_up)) continue;
+      if (!(d2 < thr2_up) || __float_as_int(q4.w) == body) continue;
       const float dist = sqrtf(d2);
       if (!(dist < thr)) continue;
+      const uint32_t kj = __ldg(skeys + j);
+      if (kj != cell) {
+        lin = ar::add(lin, cf);
+        cf = ar::mk3(0.f, 0.f, 0.f);
+        cell = kj;
+      }
       const float3 v2 = ar::xyz(__ldg(svel + j));
-      const float3 f = ar_dem::spring_force(rp, dist, ar::sub(v2, vel), thr, kk, dmp, shr, att);
-      if (t < na) fa = ar::add(fa, f);
-      else if (t < nab) fb = ar::add(fb, f);
-      else fc = ar::add(fc, f);
+      cf = ar::add(cf, ar_dem::spring_force(rp, dist, ar::sub(v2, vel), thr, S.k, S.damping, S.shear,
+                                            S.attraction));
     }
-    lin = ar::add(lin, fa);
-    lin = ar::add(lin, fb);
-    lin = ar::add(lin, fc);
   }
+  lin = ar::add(lin, cf);
   lin = ar::add(lin, ar_pipe::wall_force(S, pos, vel));
   pforce[__ldg(svals + k)] = make_float4(lin.x, lin.y, lin.z, 0.f);
 }
@@ -381,6 +390,114 @@ __device__ __forceinline__ uint32_t near_cell(const SceneDev& S, uint32_t local,
   const uint32_t y = ((local >> lx) + (uint32_t)(r / 3 % 3) - 1u) & my;
   const uint32_t z = ((local >> (lx + ly)) + (uint32_t)(r / 9) - 1u) & mz;
   return (z << (lx + ly)) + (y << lx) + x;
+}
+
+// ---- K4 for few particles: a warp walks a particle's candidates together --------------------
+// The same gather for scenes that cannot fill the chip with a thread per particle.  A warp owns
+// per_warp consecutive sorted particles (a power of two): its first per_warp lanes find their
+// particles' cells to visit, then the warp takes those particles one after another: lanes 0..26
+// load the cells' entries, a prefix sum over their counts numbers the candidates in cell order,
+// each lane tests one, and the contacts' forces are added in that order with a partial sum per
+// cell.  One thread per particle waits out a dependent round trip per row and candidate with too
+// few warps to hide it (@FEW@).
+template <bool kOne>
+__global__ void __launch_bounds__(256) collide_few_kernel(
+    const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table, int nt, int per_warp,
+    const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ svals,
+    const uint2* __restrict__ cells, const float4* __restrict__ spos,
+    const float4* __restrict__ svel, float4* __restrict__ pforce,
+    const long long* __restrict__ d_step) {
+  ar::pdl_wait();
+  const int lane = ar::lane_id();
+  const int k = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane;
+  const bool mine = lane < per_warp && k < nt;
+  const uint32_t epoch = cell_epoch(*d_step);
+  float4 p4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = p4;
+  uint32_t key = 0, todo = 0;
+  float3 lin = ar::mk3(0.f, 0.f, 0.f);
+  if (mine) {
+    p4 = __ldg(spos + k);
+    v4 = __ldg(svel + k);
+    key = __ldg(skeys + k);
+    const SceneDev& S = scene_at<kOne>(one, table, kOne ? 0 : __float_as_int(v4.w));
+    const uint32_t own = own_meta(epoch, body_tag(__float_as_int(p4.w) - S.boff));
+    const uint32_t* __restrict__ meta = reinterpret_cast<const uint32_t*>(cells) + 1;
+#pragma unroll
+    for (int r = 0; r < 27; ++r)
+      todo |= live_meta(__ldg(meta + 2 * (size_t)(S.cell_base + near_cell(S, key - S.cell_base, r))),
+                        epoch, own) << r;
+  }
+  for (uint32_t work = __ballot_sync(0xffffffffu, todo != 0); work; work &= work - 1) {
+    const int src = __ffs(work) - 1;
+    auto pick = [&](float x) { return __shfl_sync(0xffffffffu, x, src); };
+    const float3 pos = ar::mk3(pick(p4.x), pick(p4.y), pick(p4.z));
+    const float3 vel = ar::mk3(pick(v4.x), pick(v4.y), pick(v4.z));
+    const int body = __float_as_int(pick(p4.w)), sc = __float_as_int(pick(v4.w));
+    const SceneDev& S = scene_at<kOne>(one, table, kOne ? 0 : sc);
+    const uint32_t local = __shfl_sync(0xffffffffu, key, src) - S.cell_base;
+    const uint32_t visit = __shfl_sync(0xffffffffu, todo, src);
+    const float thr = 2.0f * S.r;
+    const float thr2_up = nextafterf(thr * thr, INFINITY);
+    uint32_t first = 0, count = 0;  // this lane's cell: first slot and occupants to visit
+    if ((visit >> lane) & 1u) {
+      const uint32_t cell = S.cell_base + near_cell(S, local, lane);
+      const uint2 c = __ldg(cells + cell);
+      first = c.x;
+      count = c.y & kCountMask;
+      if (count == kCountMask)  // a saturated count is resolved from the keys
+        while (c.x + count < (uint32_t)nt && __ldg(skeys + c.x + count) == cell) ++count;
+    }
+    uint32_t upto = count;  // inclusive prefix sum of the counts
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, upto, 31);
+    const uint32_t shift = first - (upto - count);  // candidate t of this cell is slot t + shift
+    float3 sum = ar::mk3(0.f, 0.f, 0.f), cf = sum;
+    int cell_now = -1;
+    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+      const uint32_t t = t0 + lane;
+      int c = 0;  // the cell that holds candidate t: the first whose prefix exceeds t
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(0xffffffffu, upto, c + o - 1) <= t) c += o;
+      const uint32_t j = t + __shfl_sync(0xffffffffu, shift, c & 31);
+      bool hit = false;
+      float3 f = ar::mk3(0.f, 0.f, 0.f);
+      if (t < total) {
+        const float4 q4 = __ldg(spos + j);
+        const float3 rp = ar::sub(ar::xyz(q4), pos);
+        const float d2 = ar::dot(rp, rp);
+        if (d2 < thr2_up && __float_as_int(q4.w) != body) {
+          const float dist = sqrtf(d2);
+          hit = dist < thr;
+          if (hit)
+            f = ar_dem::spring_force(rp, dist, ar::sub(ar::xyz(__ldg(svel + j)), vel), thr, S.k,
+                                     S.damping, S.shear, S.attraction);
+        }
+      }
+      for (uint32_t hits = __ballot_sync(0xffffffffu, hit); hits; hits &= hits - 1) {
+        const int h = __ffs(hits) - 1;
+        const int hc = __shfl_sync(0xffffffffu, c, h);
+        if (hc != cell_now) {  // cells without contacts would add +0, which changes nothing
+          sum = ar::add(sum, cf);
+          cf = ar::mk3(0.f, 0.f, 0.f);
+          cell_now = hc;
+        }
+        cf = ar::add(cf, ar::mk3(__shfl_sync(0xffffffffu, f.x, h),
+                                 __shfl_sync(0xffffffffu, f.y, h),
+                                 __shfl_sync(0xffffffffu, f.z, h)));
+      }
+    }
+    if (lane == src) lin = ar::add(sum, cf);
+  }
+  if (mine) {
+    const SceneDev& S = scene_at<kOne>(one, table, kOne ? 0 : __float_as_int(v4.w));
+    lin = ar::add(lin, ar_pipe::wall_force(S, ar::xyz(p4), ar::xyz(v4)));
+    pforce[__ldg(svals + k)] = make_float4(lin.x, lin.y, lin.z, 0.f);
+  }
 }
 
 // ---- K4b: the static point cloud of the scene ---------------------------------------------
@@ -1241,6 +1358,14 @@ void launch_resort(ar_ctx* ctx, ar_batch* B, const ar_resort::Work& rw, cudaStre
 // | sort | tree (Karras nodes, leaves, scene roots, refit) | collide | body sums + integration.
 constexpr int kStages = 6;
 
+// The gather walks with whole warps up to this many particles per SM, with at least kFewWarps
+// warps per SM.  Measured on a B200, step of packed / spread-out cubes against one thread per
+// particle: 1,728 particles 25.4 / 24.1 us against 37.8 / 24.2, 5,832: 29.9 / 25.4 against
+// 41.9 / 25.3, 13,824: 35.5 / 26.7 against 43.5 / 26.5; at 19,683 the two meet (43.4 / 26.9
+// against 43.8 / 27.0), and from 46,656 on the thread is better (61.8 against 47.4).  More warps
+// help packed scenes and hurt spread-out ones (16 per SM: 13,824 in 33.7 / 27.9 us).
+constexpr int kFewPerSm = 96;
+constexpr int kFewWarps = 8;
 // The cloud kernel: a particle near the cloud costs its warp thousands of points, so it spreads
 // the particles over more warps.
 constexpr int kCloudWarps = 32;
@@ -1362,8 +1487,15 @@ ar_status enqueue_step(ar_batch* B, cudaStream_t st, cudaEvent_t* ev = nullptr) 
   AR_LAUNCH_ONE(scatter_kernel, dim3(gp), dim3(256), B->d_table, B->d_pscene, nt, B->skeys,
       B->svals, B->cells, B->spos, B->svel, B->pkeys, B->pvals, B->d_step);
   mark(4);
-  AR_LAUNCH_ONE(collide_kernel, dim3(arh::grid_for(nt, bs)), dim3(bs), B->d_table, nt,
-      B->skeys, B->svals, B->cells, B->spos, B->svel, B->pforce, B->d_step);
+  if (nt <= ctx->num_sms * kFewPerSm) {
+    const int per_warp = per_warp_for(ctx, nt, kFewWarps);
+    AR_LAUNCH_ONE(collide_few_kernel, dim3(arh::grid_for(nt, bs / 32 * per_warp)), dim3(bs),
+        B->d_table, nt, per_warp, B->skeys, B->svals, B->cells, B->spos, B->svel, B->pforce,
+        B->d_step);
+  } else {
+    AR_LAUNCH_ONE(collide_kernel, dim3(arh::grid_for(nt, bs)), dim3(bs), B->d_table, nt,
+        B->skeys, B->svals, B->cells, B->spos, B->svel, B->pforce, B->d_step);
+  }
   if (B->has_cloud) {
     const int per_warp = per_warp_for(ctx, nt, kCloudWarps);
     AR_LAUNCH_ONE(cloud_collide_kernel, dim3(arh::grid_for(nt, 4 * per_warp)), dim3(128),

@@ -92,7 +92,7 @@ def stage_bytes_bvh(n: int, nb: int, passes: int, key_bits: int = 64) -> dict[st
     tiles = (n + 8191) // 8192
     k32 = key_bits <= 32
     return {
-        "clear": 4 * n + (4 * (4 + 2 * 4096) if k32 else 0),  # refit arrival counters
+        "clear": 4 * (4 + 2 * 4096) if k32 else 0,  # the re-sort's counters
         # rel in, key out; body pose per body
         "keys": n * (16 + (4 if k32 else 8)) + nb * 32,
         # re-sort: previous keys + indices in, new key gathered, mover bits; placement: previous
@@ -100,11 +100,10 @@ def stage_bytes_bvh(n: int, nb: int, passes: int, key_bits: int = 64) -> dict[st
         # first pass reads keys, every pass writes key + index, later passes read both
         "sort": (n * (8 + 4 + 0.125) + n * (8 + 0.125 + 8) + (n // 2048) * 40) if k32 else
                 n * 8 + n * (8 + 12) + (passes - 1) * n * 24 + passes * 4 * 512 * tiles,
-        # nodes: keys in, flags, children, parent, ranges and wide-node ids out; leaves: index,
-        # rel in, sorted pos + vel and the leaf box out (and the order kept, 32-bit keys), body
-        # state per body; refit: links and the node's two child boxes in, its box out
-        "tree": n * ((4 if k32 else 8) + 21 + 8 + 8) + n * (4 + 16 + 32 + 24 + 9) +
-                (n * 8 if k32 else 0) + nb * BODY_STATE + n * (8 + 64 + 24),
+        # keys, index and rel in, body state per body; sorted pos + vel out (and the order kept,
+        # 32-bit keys); links and the wide node out
+        "tree": n * ((4 if k32 else 8) + 4 + 16 + 32) + (n * 8 if k32 else 0) +
+                nb * BODY_STATE + n * (16 + 64),
         # own index, position + velocity in; force out
         "collide": n * (4 + 32 + 16),
         "body": n * (16 + 16) + _body_bytes(nb),
@@ -428,9 +427,9 @@ def run_ours(args):
             cpu_baseline = {"value": rate / 1e6, "unit": "Mparticle-steps/s", "cores": cores,
                             "kind": kind, "sample": sample, "semantics": REFERENCE_SEMANTICS}
 
-    # memset nodes are not kernels: the BVH step has two (refit counters, sort head), the grid
-    # step none (its clears are a kernel)
-    memsets = 2 if args.broadphase == "bvh" else 0
+    # memset nodes are not kernels: the BVH step has one (sort head), the grid step none (its
+    # clears are a kernel)
+    memsets = 1 if args.broadphase == "bvh" else 0
     launches = args.steps * (gs.launches_per_step() - memsets)
     if rank == 0:
         line = {

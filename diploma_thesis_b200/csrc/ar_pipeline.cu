@@ -20,13 +20,13 @@
 // scene and within a scene exactly as a solo sort would: batched and solo steps are
 // bit-identical.  The sequence is captured once into a CUDA graph and replayed.
 //
-// Batches of BVH scenes replace K0-K4 by: a memset of the refit's arrival counters; Morton keys
+// Batches of BVH scenes replace K0-K4 by: Morton keys
 // (scene index above the particle's 30-bit code: 32-bit keys for up to 4 scenes, else 64-bit);
 // the sort (32-bit keys re-sorted from the last step's order as above, 64-bit keys radix-sorted
-// every step); Karras nodes over all scenes (equal codes tie-broken by the index within the
-// scene); leaves in sorted order, each leaf's thread then climbing the refit (acquire-release
-// arrival counters); each scene's subtree root; and per particle a walk of its scene's subtree
-// in the reference's visit order with a 64-entry stack.  K5 is shared.
+// every step); one kernel for the tree over all scenes (equal codes tie-broken by the index
+// within the scene): leaves, nodes with their boxes, each scene's subtree root (ar_tree.cuh); and
+// per particle a walk of its scene's subtree in the reference's visit order with a 64-entry
+// stack.  K5 is shared.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -39,6 +39,7 @@
 #include "ar_pipeline.cuh"
 #include "ar_resort.cuh"
 #include "ar_sort.cuh"
+#include "ar_tree.cuh"
 
 using ar_pipe::SceneDev;
 
@@ -671,145 +672,95 @@ struct __align__(64) WideNode {
   float4 c[4];
 };
 
-__device__ __forceinline__ int* node_ints(WideNode* nodes, int internal) {
-  return reinterpret_cast<int*>(nodes + internal);
-}
-// Box, id and body tag of child `side` (0 left, 1 right) into the parent's slot.
-__device__ __forceinline__ void put_child(WideNode* nodes, int internal, int side, float4 lo,
-                                          float2 hi_yz, int id, int tag) {
-  float4* c = nodes[internal].c + 2 * side;
-  __stcg(c, lo);
-  __stcg(c + 1, make_float4(hi_yz.x, hi_yz.y, __int_as_float(id), __int_as_float(tag)));
-}
-
-template <class Lcp>
-__global__ void __launch_bounds__(256) bvh_build_kernel(Lcp lcp, int n,
-                                                        uint8_t* __restrict__ is_leaf,
-                                                        int32_t* __restrict__ left,
-                                                        int32_t* __restrict__ right,
-                                                        int32_t* __restrict__ parent,
-                                                        int32_t* __restrict__ min_r,
-                                                        int32_t* __restrict__ max_r,
-                                                        WideNode* __restrict__ nodes) {
-  ar::pdl_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) parent[n] = -1;
-  if (i >= n - 1) return;
-  ar_lbvh::karras_node(i, n, lcp, is_leaf, left, right, parent, min_r, max_r);
-}
-
-// Bottom-up refit (kernelConstructInternalNodesSoA, BVHSource/BVHSoAKernels.cu:148-176) from
-// one leaf whose box is already in its parent's slot (ar_lbvh::refit_climb): the second thread
-// to reach a node merges the two child boxes held in the node (mergeBounds,
-// BVHAuxiliary.cuh:83-94) and stores the result, with the merged body tag, into the node's slot
-// in its parent, then climbs on.  Release / acquire through the arrival counter; boxes through
-// L2.
-__device__ __forceinline__ void refit_from_leaf(int i, int n, const int32_t* __restrict__ left,
-                                                const int32_t* __restrict__ parent,
-                                                WideNode* nodes, int* __restrict__ counters) {
-  // The climb of ar_lbvh::refit_climb with the wide nodes: the second child to arrive at a node
-  // merges the node's two child records (boxes, and body tags in their w) and writes the result
-  // into the node's slot in its parent.  The parent and the side of the slot depend only on
-  // the tree, so they are loaded before the arrival: each level costs the arrival and the
-  // children's records, two round trips.
-  int node = __ldg(parent + i);
-  if (node < n || node >= 2 * n - 1) return;  // malformed parent link
-  int pn = node != n ? __ldg(parent + node) : n;
-  int side = node != n ? (__ldg(left + pn) == node ? 0 : 1) : 0;
-  for (int depth = 0; depth < n; ++depth) {  // a valid tree is at most n - 1 deep
-    // the next level's parent and side, loaded while the arrival is in flight (wasted when this
-    // thread arrives first)
-    const int next = pn;
-    const bool next_ok = next != n && next >= n && next < 2 * n - 1;
-    const int npn = next_ok ? __ldg(parent + next) : n;
-    if (ar_lbvh::arrive(counters + (node - n)) == 0) return;
-    const float4* c = nodes[node - n].c;
-    const float4 a0 = __ldcg(c), a1 = __ldcg(c + 1), b0 = __ldcg(c + 2), b1 = __ldcg(c + 3);
-    if (node == n) return;  // the root's box is not stored anywhere
-    if (next != n && !next_ok) return;  // malformed parent link
-    const int nside = next_ok && npn >= n && npn < 2 * n - 1 && __ldg(left + npn) != next ? 1 : 0;
-    const ar_lbvh::Box6 m = ar_lbvh::merge_boxes(ar_lbvh::Box6{a0.x, a0.y, a0.z, a0.w, a1.x, a1.y},
-                                                 ar_lbvh::Box6{b0.x, b0.y, b0.z, b0.w, b1.x, b1.y});
-    // both children have arrived, so their tags (the records' last words) are visible like
-    // their boxes
-    const int tl = __float_as_int(a1.w), tr = __float_as_int(b1.w);
-    put_child(nodes, pn - n, side, make_float4(m.lx, m.ly, m.lz, m.hx), make_float2(m.hy, m.hz),
-              node, tl == tr ? tl : -1);
-    node = next;
-    pn = npn;
-    side = nside;
-  }
-}
-
-// Leaves in sorted order: position (w = global body id) and velocity recomputed from the body
-// state; the leaf box (position +/- r) goes into its parent's slot, and the thread climbs from
-// there (the refit); leaf flags and ranges.
+// Where a step's tree goes: links in the reference's numbering, wide nodes, each scene's root.
+// A node whose leaves share the key bits above the Morton code, but not with its neighbours, is
+// its scene's root.
 template <bool kOne>
-__global__ void __launch_bounds__(256) bvh_leaves_kernel(
-    const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table, const int* __restrict__ pscene, int ns, int nt,
-    const uint32_t* __restrict__ svals, const int32_t* __restrict__ left,
-    const int32_t* __restrict__ parent, float4* __restrict__ spos, float4* __restrict__ svel,
-    WideNode* __restrict__ nodes, uint8_t* __restrict__ is_leaf, int32_t* __restrict__ min_r,
-    int32_t* __restrict__ max_r, int* __restrict__ counters, const uint32_t* __restrict__ skeys32,
-    uint32_t* __restrict__ prev_keys, uint32_t* __restrict__ prev_vals) {
+struct StepTree {
+  static constexpr bool kBoxes = true;
+  int32_t *left, *right, *parent, *roots;
+  WideNode* nodes;
+  const float4 *spos, *svel;
+  const SceneDev* one;
+  const SceneDev* table;
+  int prefix;  // key bits above the Morton code
+
+  __device__ __forceinline__ int scene_of(int leaf) const {
+    return kOne ? 0 : __float_as_int(__ldcg(svel + leaf).w);
+  }
+  __device__ __forceinline__ static ar_tree::Box2 record(float3 p, float r, int leaf, int tag) {
+    return ar_tree::Box2{make_float4(p.x - r, p.y - r, p.z - r, p.x + r),
+                         make_float4(p.y + r, p.z + r, __int_as_float(leaf), __int_as_float(tag))};
+  }
+  __device__ __forceinline__ ar_tree::Box2 leaf(int i) const {
+    const float4 p = __ldcg(spos + i);
+    return record(ar::xyz(p), scene_at<kOne>(*one, table, scene_of(i)).r, i, __float_as_int(p.w));
+  }
+  __device__ __forceinline__ void made(int id, int d, int dl, int dr, int first, int) const {
+    if (d >= prefix && dl < prefix && dr < prefix) roots[scene_of(first)] = id;
+  }
+  __device__ __forceinline__ void links(int id, int lc, int rc, int, int) const {
+    left[id] = lc;
+    right[id] = rc;
+  }
+  __device__ __forceinline__ void parent_of(int child, int id) const { parent[child] = id; }
+  __device__ __forceinline__ void wide(int number, int part, float4 v) const {
+    nodes[number].c[part] = v;
+  }
+};
+
+// The whole tree of a step from the sorted keys (ar_tree.cuh): the leaves' positions and
+// velocities from the body state, then the nodes with their boxes (kernelConstructRadixTreeSoA,
+// kernelConstructLeafNodesSoA and kernelConstructInternalNodesSoA, BVHSource/BVHSoAKernels.cu:
+// 7-176; boxes merged left child first by mergeBounds, BVHAuxiliary.cuh:83-94).
+// One launch in place of a build that searched each node's range from global memory, leaves that
+// climbed with a device-scope arrival per node, and a root search (2M pile: 275 -> 184 us; 12
+// scenes, 290k particles, 64-bit keys: 91 -> 62 us).  Bound by latency and issue: 1,200 warp
+// instructions per 32 leaves, half of the issue slots used, then about 45 us of the last groups'
+// levels with most SMs idle.  Tiles of 128 (217 us) leave twice the subtrees to the levels above;
+// groups of 8 or 32 lists add a level or a tile to each (197, 236 us); finishing the nodes in
+// block-wide rounds instead of the climb executed 30 % more instructions.
+template <class Lcp, bool kOne>
+__global__ void __launch_bounds__(ar_tree::kTile, 6) bvh_tree_kernel(
+    const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table,
+    const int* __restrict__ pscene, int n, Lcp lcp, const uint32_t* __restrict__ svals,
+    float4* spos, float4* svel, StepTree<kOne> out, ar_tree::Scratch work,
+    const uint32_t* __restrict__ skeys32, uint32_t* __restrict__ prev_keys,
+    uint32_t* __restrict__ prev_vals) {
+  constexpr int kT = ar_tree::kTile;
+  __shared__ ar_tree::Links s;
+  __shared__ ar_tree::Boxes box;
   ar::pdl_wait();
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) {
+  out.one = &one;
+  const int t = threadIdx.x, base = blockIdx.x * kT, m = min(kT, n - base), k = base + t;
+  ar_tree::reset_links(s);
+  if (t < m) {
     const int g = (int)__ldg(svals + k);
     if (prev_keys) {  // 32-bit keys: the order the next step's re-sort starts from
       prev_keys[k] = __ldg(skeys32 + k);
       prev_vals[k] = (uint32_t)g;
     }
-    const int sc = kOne ? 0 : __ldg(pscene + g);
-    const SceneDev& S = scene_at<kOne>(one, table, sc);
+    const int scene = kOne ? 0 : __ldg(pscene + g);
+    const SceneDev& S = scene_at<kOne>(one, table, scene);
     const float4 r4 = __ldg(S.rel + (g - S.poff));
     const int b = __float_as_int(r4.w);
     float3 r, p, v;
     ar_pipe::repose(__ldg(S.quat + b), __ldg(S.pos + b), __ldg(S.vel + b), __ldg(S.ang + b),
                     ar::mk3(r4.x, r4.y, r4.z), &r, &p, &v);
     spos[k] = make_float4(p.x, p.y, p.z, __int_as_float(S.boff + b));
-    svel[k] = make_float4(v.x, v.y, v.z, __int_as_float(sc));  // w = scene index
-    if (nt >= 2) {
-      const float rr = S.r;
-      const int pn = __ldg(parent + k);
-      put_child(nodes, pn - nt, __ldg(left + pn) == k ? 0 : 1,
-                make_float4(p.x - rr, p.y - rr, p.z - rr, p.x + rr), make_float2(p.y + rr, p.z + rr),
-                k, S.boff + b);
-      refit_from_leaf(k, nt, left, parent, nodes, counters);  // the climb starts right here
-    }
-    is_leaf[k] = 1;
-    min_r[k] = k;
-    max_r[k] = k;
+    svel[k] = make_float4(v.x, v.y, v.z, __int_as_float(scene));  // w = scene index
+    const ar_tree::Box2 rec = StepTree<kOne>::record(p, S.r, k, S.boff + b);
+    box.a[t] = rec.a;
+    box.b[t] = rec.b;
+    s.first[t] = s.last[t] = s.id[t] = k;
+    s.d[0][t] = (signed char)lcp(k, k - 1);
+    if (t == m - 1) s.d[0][m] = (signed char)lcp(k, k + 1);
   }
-}
-
-// Each scene's subtree root.  The scene's leaves [lo, hi] are one subtree, whose root covers
-// exactly [lo, hi]; a Karras internal node i has i as one end of its range, so the root is
-// internal node lo or internal node hi.  (The walk up from the first leaf is kept only as a
-// guard against a malformed tree.)
-__global__ void bvh_roots_kernel(const int* __restrict__ poff, int ns, int nt,
-                                 const int32_t* __restrict__ parent,
-                                 const int32_t* __restrict__ min_r,
-                                 const int32_t* __restrict__ max_r, int32_t* __restrict__ roots) {
-  ar::pdl_wait();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= ns) return;
-  const int lo = poff[s], hi = poff[s + 1] - 1;
-  if (hi <= lo) {  // zero or one particle: no internal node
-    roots[s] = -1;
-    return;
-  }
-  for (const int cand : {nt + lo, nt + hi}) {
-    if (cand <= 2 * nt - 2 && min_r[cand] == lo && max_r[cand] == hi) {
-      roots[s] = cand;
-      return;
-    }
-  }
-  int node = parent[lo];
-  for (int depth = 0; depth < nt && node >= 0; ++depth) {
-    if (min_r[node] <= lo && max_r[node] >= hi) break;
-    node = parent[node];
-  }
-  roots[s] = node;
+  if (k == 0) out.parent[n] = -1;
+  __syncthreads();
+  if (t < m && s.d[0][t] < out.prefix && s.d[0][t + 1] < out.prefix)
+    out.roots[out.scene_of(k)] = -1;  // a scene of one particle
+  ar_tree::build_up(s, &box, m, n, lcp, out, work);
 }
 
 // DEM gather through the scene's subtree in the reference's visit order
@@ -1059,11 +1010,9 @@ struct ar_batch {
   long cap_bvh = 0;
   size_t cap_sort64 = 0;
   uint64_t *keys64 = nullptr, *skeys64 = nullptr;
-  uint8_t* is_leaf = nullptr;
-  int32_t *left = nullptr, *right = nullptr, *parent = nullptr, *min_r = nullptr,
-          *max_r = nullptr, *roots = nullptr;
+  int32_t *left = nullptr, *right = nullptr, *parent = nullptr, *roots = nullptr;
   WideNode* nodes = nullptr;
-  int* counters = nullptr;
+  ar_tree::Scratch tree{};
   char* sort64_ws = nullptr;
   int bvh_key_bits = kMortonBits;
   // graph
@@ -1094,14 +1043,14 @@ void free_batch_buffers(ar_batch* B) {
   B->cap_n = B->cap_b = B->cap_s = 0;
   B->cap_cells = 0;
   B->cap_sort = 0;
-  cudaFree(B->keys64); cudaFree(B->skeys64); cudaFree(B->is_leaf); cudaFree(B->left);
-  cudaFree(B->right); cudaFree(B->parent); cudaFree(B->min_r); cudaFree(B->max_r);
-  cudaFree(B->roots); cudaFree(B->nodes); cudaFree(B->counters); cudaFree(B->sort64_ws);
+  cudaFree(B->keys64); cudaFree(B->skeys64); cudaFree(B->left); cudaFree(B->right);
+  cudaFree(B->parent); cudaFree(B->roots); cudaFree(B->nodes); cudaFree(B->tree.open);
+  cudaFree(B->tree.pending); cudaFree(B->tree.length); cudaFree(B->tree.arrived);
+  cudaFree(B->sort64_ws);
   B->keys64 = B->skeys64 = nullptr;
-  B->is_leaf = nullptr;
-  B->left = B->right = B->parent = B->min_r = B->max_r = B->roots = nullptr;
+  B->left = B->right = B->parent = B->roots = nullptr;
   B->nodes = nullptr;
-  B->counters = nullptr;
+  B->tree = ar_tree::Scratch{};
   B->sort64_ws = nullptr;
   B->cap_bvh = 0;
   B->cap_sort64 = 0;
@@ -1246,13 +1195,16 @@ ar_status prepare(ar_batch* B, cudaStream_t st) {
       const long cn = B->cap_n;
       const size_t m = 2 * (size_t)cn;
       const size_t csort = ar_sort::layout(cn, 8, passes64).total;
-      cudaFree(B->keys64); cudaFree(B->skeys64); cudaFree(B->is_leaf); cudaFree(B->left);
-      cudaFree(B->right); cudaFree(B->parent); cudaFree(B->min_r); cudaFree(B->max_r);
-      cudaFree(B->roots); cudaFree(B->nodes); cudaFree(B->counters); cudaFree(B->sort64_ws);
-      bool ok = alloc(&B->keys64, cn) && alloc(&B->skeys64, cn) && alloc(&B->is_leaf, m) &&
-                alloc(&B->left, m) && alloc(&B->right, m) && alloc(&B->parent, m) &&
-                alloc(&B->min_r, m) && alloc(&B->max_r, m) && alloc(&B->roots, B->cap_s) &&
-                alloc(&B->nodes, cn) && alloc(&B->counters, cn) &&
+      cudaFree(B->keys64); cudaFree(B->skeys64); cudaFree(B->left); cudaFree(B->right);
+      cudaFree(B->parent); cudaFree(B->roots); cudaFree(B->nodes); cudaFree(B->tree.open);
+      cudaFree(B->tree.pending); cudaFree(B->tree.length); cudaFree(B->tree.arrived);
+      cudaFree(B->sort64_ws);
+      const size_t lists = ar_tree::lists_for(cn);
+      bool ok = alloc(&B->keys64, cn) && alloc(&B->skeys64, cn) && alloc(&B->left, m) &&
+                alloc(&B->right, m) && alloc(&B->parent, m) && alloc(&B->roots, B->cap_s) &&
+                alloc(&B->nodes, cn) && alloc(&B->tree.open, cn) &&
+                alloc(&B->tree.pending, 2 * cn) && alloc(&B->tree.length, lists) &&
+                alloc(&B->tree.arrived, lists) &&
                 alloc(&B->sort64_ws, csort);
       if (!ok) {
         free_batch_buffers(B);
@@ -1261,6 +1213,7 @@ ar_status prepare(ar_batch* B, cudaStream_t st) {
       }
       B->cap_bvh = cn;
       B->cap_sort64 = csort;
+      cudaMemsetAsync(B->tree.arrived, 0, lists * sizeof(int), st);
     }
   }
   if (ns > 0) {
@@ -1352,10 +1305,23 @@ void launch_resort(ar_ctx* ctx, ar_batch* B, const ar_resort::Work& rw, cudaStre
       ctx->d_err);
 }
 
+// The tree of a BVH step.  32-bit keys leave this step's order for the next step's re-sort.
+template <bool kOne, class Lcp>
+void launch_tree(ar_batch* B, const Lcp& lcp, int prefix, cudaStream_t st) {
+  const int nt = (int)B->nt;
+  const bool keep = B->bvh_key_bits <= 32;
+  const StepTree<kOne> out{B->left, B->right, B->parent, B->roots, B->nodes, B->spos, B->svel,
+                           nullptr, B->d_table, prefix};
+  arh::launch_pdl(bvh_tree_kernel<Lcp, kOne>, dim3(arh::grid_for(nt, ar_tree::kTile)),
+      dim3(ar_tree::kTile), 0, st, B->one, B->d_table, B->d_pscene, nt, lcp, B->svals, B->spos,
+      B->svel, out, B->tree, (const uint32_t*)B->skeys, keep ? B->pkeys : nullptr,
+      keep ? B->pvals : nullptr);
+}
+
 // Stage boundaries for ar_step_profile: events[0] before the step, events[i] after stage i.
 // Grid: clear (sort histogram head, cell-table slice) | cell keys + histogram | sort |
-// scatter + cell table | collide | body sums + integration.  BVH: clear (refit counters) | Morton keys
-// | sort | tree (Karras nodes, leaves, scene roots, refit) | collide | body sums + integration.
+// scatter + cell table | collide | body sums + integration.  BVH: nothing | Morton keys
+// | sort | tree (leaves, nodes, boxes, scene roots) | collide | body sums + integration.
 constexpr int kStages = 6;
 
 // The gather walks with whole warps up to this many particles per SM, with at least kFewWarps
@@ -1399,7 +1365,6 @@ ar_status enqueue_step(ar_batch* B, cudaStream_t st, cudaEvent_t* ev = nullptr) 
   } while (0)
   mark(0);
   if (B->broadphase == AR_BROADPHASE_BVH) {
-    cudaMemsetAsync(B->counters, 0, (size_t)nt * sizeof(int), st);  // refit arrival counters
     mark(1);
     // keys of at most 32 bits (up to 4 scenes) are sorted as uint32: half the bytes per pass
     const bool k32 = B->bvh_key_bits <= 32;
@@ -1428,23 +1393,11 @@ ar_status enqueue_step(ar_batch* B, cudaStream_t st, cudaEvent_t* ev = nullptr) 
       if (s != AR_OK) return s;
     }
     mark(3);
-    const dim3 gb(arh::grid_for(std::max(nt - 1, 1), 256));
-    if (k32)
-      arh::launch_pdl(bvh_build_kernel<ar_lbvh::Lcp32Scene>, gb, dim3(256), 0, st,
-          ar_lbvh::Lcp32Scene{B->skeys, nt, B->d_poff, kMortonBits}, nt, B->is_leaf, B->left,
-          B->right, B->parent, B->min_r, B->max_r, B->nodes);
-    else
-      arh::launch_pdl(bvh_build_kernel<ar_lbvh::Lcp64Scene>, gb, dim3(256), 0, st,
-          ar_lbvh::Lcp64Scene{B->skeys64, nt, B->d_poff, kMortonBits}, nt, B->is_leaf, B->left,
-          B->right, B->parent, B->min_r, B->max_r, B->nodes);
-    // one thread per leaf: each climbs after storing its leaf (128-thread blocks: a block holds
-    // its SM slot until its last climber is done; 2M pile tree stage 288 -> 278 us against 256)
-    AR_LAUNCH_ONE(bvh_leaves_kernel, dim3(arh::grid_for(nt, 128)), dim3(128), B->d_table,
-        B->d_pscene, ns, nt, B->svals, B->left, B->parent, B->spos, B->svel, B->nodes, B->is_leaf,
-        B->min_r, B->max_r, B->counters, (const uint32_t*)B->skeys, k32 ? B->pkeys : nullptr,
-        k32 ? B->pvals : nullptr);
-    arh::launch_pdl(bvh_roots_kernel, dim3(arh::grid_for(ns, 128)), dim3(128), 0, st, B->d_poff, ns,
-        nt, B->parent, B->min_r, B->max_r, B->roots);
+    const ar_lbvh::Lcp32Scene lcp32{B->skeys, nt, B->d_poff, kMortonBits};
+    const ar_lbvh::Lcp64Scene lcp64{B->skeys64, nt, B->d_poff, kMortonBits};
+    if (k32 && one) launch_tree<true>(B, lcp32, 32 - kMortonBits, st);
+    else if (k32) launch_tree<false>(B, lcp32, 32 - kMortonBits, st);
+    else launch_tree<false>(B, lcp64, 64 - kMortonBits, st);
     mark(4);
     AR_LAUNCH_ONE(bvh_collide_kernel, dim3(arh::grid_for(nt, bs)), dim3(bs), B->d_table,
         B->d_poff, ns, nt, B->svals, B->spos, B->svel, B->nodes, B->roots, B->pforce, ctx->d_err);
@@ -2162,12 +2115,11 @@ ar_status ar_scene_model_matrices(ar_scene* s, float* d_model16, ar_stream_t str
 
 int ar_batch_launches_per_step(ar_batch* B) {
   if (!B) return 0;
-  // BVH: memset, keys, the sort (32-bit keys: memset + four re-sort kernels after the first
-  // step; 64-bit keys: the radix sort), three tree kernels (build, leaves + refit, roots),
-  // collide, body sums, integration
+  // BVH: keys, the sort (32-bit keys: memset + four re-sort kernels after the first step; 64-bit
+  // keys: the radix sort), the tree, collide, body sums, integration
   if (B->broadphase == AR_BROADPHASE_BVH)
-    return 1 + 1 + (B->bvh_key_bits <= 32 ? 1 + 4 : ar_sort::launches(0, B->bvh_key_bits, false)) +
-           3 + 1 + 2;
+    return 1 + (B->bvh_key_bits <= 32 ? 1 + 4 : ar_sort::launches(0, B->bvh_key_bits, false)) +
+           1 + 1 + 2;
   // a step that re-sorts from the previous order (every step but the first after a change of
   // the member list): clear, keys, four re-sort kernels, scatter, collide (and the static
   // clouds' impulses when a scene has one), body sums, integration

@@ -745,7 +745,7 @@ AR_API ar_status ar_step(ar_ctx* ctx, ar_scene* scene, int n_steps, int use_grap
 /* Run n_steps of the scene without a graph, with CUDA events between the stages, and return
  * the average device milliseconds per stage in h_stage_ms[6].  Grid: clear (sort histogram
  * head), re-pose + cell keys + histogram, sort, scatter + cell table, DEM gather + walls, body
- * sums + integration (+ cell reset).  BVH: clear (refit counters), Morton keys, sort, tree
+ * sums + integration (+ cell reset).  BVH: nothing, Morton keys, sort, tree
  * (build, leaves, scene roots, refit), DEM traversal + walls, body sums + integration.
  * (Replaces the reference's clock() accumulators, e.g.
  * RigidBodies/UniformGridUpdate.cpp:338-446.) */

@@ -48,8 +48,16 @@ __global__ void __launch_bounds__(256) reorder_kernel(const uint32_t* __restrict
   }
 }
 
-// FindAndHandleRigidBodyCollisionsUniformGridKernel (RigidBodies/UniformGridDEM.cu:133-204).
-__global__ void __launch_bounds__(128) collide_grid_kernel(
+// FindAndHandleRigidBodyCollisionsUniformGridKernel (RigidBodies/UniformGridDEM.cu:133-204).  An
+// occupant is tested for distance first, since most fail that.  Those within reach go to a short
+// list per thread, and their bodies, which take two dependent loads, and forces are looked at from
+// the lists: in the search nearly every candidate is within reach of some lane, and the warp would
+// issue the force's two hundred instructions for each (373,248 packed particles: 130 -> 85
+// us).
+constexpr int kGridThreads = 128;
+constexpr int kHits = 16;                  // listed contacts per thread
+constexpr uint32_t kNewCell = 0x80000000u; // on the first contact of a cell; slots are below 2^31
+__global__ void __launch_bounds__(kGridThreads) collide_grid_kernel(
     ar_sim_params prm, ar_grid::Grid g, const int32_t* __restrict__ rb_idx,
     const float4* __restrict__ spos, const float4* __restrict__ svel,
     const float4* __restrict__ rel, const uint32_t* __restrict__ gidx,
@@ -63,31 +71,41 @@ __global__ void __launch_bounds__(128) collide_grid_kernel(
   const uint32_t orig = __ldg(gidx + index);
   const int body = __ldg(rb_idx + orig);
   const float thr = 2.0f * prm.particle_radius;
-  float3 lin = ar::mk3(0.f, 0.f, 0.f);
-  for (int z = -1; z <= 1; ++z)
-    for (int y = -1; y <= 1; ++y)
-      for (int x = -1; x <= 1; ++x) {
-        float3 cell_f = ar::mk3(0.f, 0.f, 0.f);
-        const uint32_t h = g.hash(make_int3(gp.x + x, gp.y + y, gp.z + z));
-        const uint32_t st = __ldg(cstart + h);
-        if (st != ar::kEmpty) {
-          const uint32_t en = __ldg(cend + h);
-          for (uint32_t j = st; j < en; ++j) {
-            const int b2 = __ldg(rb_idx + __ldg(gidx + j));
-            if (j == (uint32_t)index || body == b2) continue;
-            const float3 p2 = ar::xyz(__ldg(spos + j));
-            const float3 rp = ar::sub(p2, pos);
-            const float dist = sqrtf(ar::dot(rp, rp));
-            if (dist < thr) {
-              const float3 v2 = ar::xyz(__ldg(svel + j));
-              cell_f = ar::add(cell_f, ar_dem::spring_force(rp, dist, ar::sub(v2, vel), thr,
-                                                            prm.spring, prm.damping, prm.shear,
-                                                            prm.attraction));
-            }
-          }
-        }
+  const float thr2_up = nextafterf(thr * thr, INFINITY);
+  __shared__ uint32_t s_hits[kHits][kGridThreads];
+  float3 lin = ar::mk3(0.f, 0.f, 0.f), cell_f = lin;
+  int hits = 0;
+  // the listed contacts' forces, in order; a cell's partial sum joins the total when the next
+  // cell's first contact comes (cells without contacts would add +0, which changes nothing)
+  auto add_hits = [&]() {
+    for (int i = 0; i < hits; ++i) {
+      const uint32_t e = s_hits[i][threadIdx.x], j = e & ~kNewCell;
+      if (e & kNewCell) {
         lin = ar::add(lin, cell_f);
+        cell_f = ar::mk3(0.f, 0.f, 0.f);
       }
+      if (__ldg(rb_idx + __ldg(gidx + j)) == body) continue;
+      const float3 rp = ar::sub(ar::xyz(__ldg(spos + j)), pos);
+      const float3 v2 = ar::xyz(__ldg(svel + j));
+      cell_f = ar::add(cell_f, ar_dem::spring_force(rp, sqrtf(ar::dot(rp, rp)), ar::sub(v2, vel),
+                                                    thr, prm.spring, prm.damping, prm.shear,
+                                                    prm.attraction));
+    }
+    hits = 0;
+  };
+  ar_grid::for_occupied(g, gp, cstart, cend, [&](uint32_t st, uint32_t en) {
+    uint32_t mark = kNewCell;
+    for (uint32_t j = st; j < en; ++j) {
+      const float3 rp = ar::sub(ar::xyz(__ldg(spos + j)), pos);
+      const float d2 = ar::dot(rp, rp);
+      if (!(d2 < thr2_up) || !(sqrtf(d2) < thr) || j == (uint32_t)index) continue;
+      s_hits[hits++][threadIdx.x] = j | mark;
+      mark = 0;
+      if (hits == kHits) add_hits();
+    }
+  });
+  add_hits();
+  lin = ar::add(lin, cell_f);
   float4 f = p_force[orig];
   p_force[orig] = make_float4(f.x + lin.x, f.y + lin.y, f.z + lin.z, f.w + 0.f);
   const float3 t = ar::cross(ar::xyz(__ldg(rel + orig)), lin);
@@ -292,7 +310,7 @@ ar_status ar_collide_grid_dem(ar_ctx* ctx, const ar_sim_params* params, const in
   ar_grid::Grid g;
   ar_status s = grid_from_params(params, &g);
   if (s != AR_OK || n == 0) return s;
-  collide_grid_kernel<<<arh::grid_for(n, 128), 128, 0, arh::stream(stream)>>>(
+  collide_grid_kernel<<<arh::grid_for(n, kGridThreads), kGridThreads, 0, arh::stream(stream)>>>(
       *params, g, rb_idx, (const float4*)sorted_pos4, (const float4*)sorted_vel4,
       (const float4*)rel4, grid_idx, cell_start, cell_end, n, (float4*)p_force4,
       (float4*)p_torque4);

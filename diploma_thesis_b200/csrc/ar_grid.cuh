@@ -30,4 +30,45 @@ struct Grid {
   }
 };
 
+// Calls visit(first, end) for every occupied cell among the 27 around `c`, in z, y, x order, with
+// its range of sorted slots.  The cell starts of a row are loaded one row ahead; empty cells are
+// passed over (a float sum that starts at +0 is never -0, so the +0 that an empty cell would add
+// changes nothing).  All lanes of a warp look at the same neighbour at a time, so that their
+// loads, like their cells, lie side by side: letting each lane jump to its next occupied cell
+// scattered the loads and was slower.
+template <class Visit>
+__device__ __forceinline__ void for_occupied(const Grid& g, int3 c,
+                                             const uint32_t* __restrict__ cell_start,
+                                             const uint32_t* __restrict__ cell_end, Visit visit) {
+  uint32_t x[3], start[3], next[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) x[i] = (uint32_t)(c.x + i - 1) & (g.gx - 1);
+  auto row_of = [&](int dz, int dy) {
+    return (((uint32_t)(c.z + dz) & (g.gz - 1)) * g.gy + ((uint32_t)(c.y + dy) & (g.gy - 1))) * g.gx;
+  };
+  uint32_t row = row_of(-1, -1);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) next[i] = __ldg(cell_start + row + x[i]);
+  for (int dz = -1, dy = -1; dz <= 1;) {
+    const uint32_t here = row;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) start[i] = next[i];
+    if (++dy > 1) {
+      dy = -1;
+      ++dz;
+    }
+    if (dz <= 1) {
+      row = row_of(dz, dy);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) next[i] = __ldg(cell_start + row + x[i]);
+    }
+    uint32_t end[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) end[i] = start[i] != ar::kEmpty ? __ldg(cell_end + here + x[i]) : 0u;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (start[i] != ar::kEmpty) visit(start[i], end[i]);
+  }
+}
+
 }  // namespace ar_grid

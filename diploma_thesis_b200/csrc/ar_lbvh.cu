@@ -4,11 +4,12 @@
 // i, internal node i at n + i, root at n.  Boxes are the reference's 32-byte AABB
 // {min.xyz, max.xyz, pad, pad}, read as two float4.
 //
-// Traversal is stackless: the tree's parent links replace the reference's int[64] stack.
-// The visit order is the reference's (RB_BVHKernels.cu:145-214): at an internal node, its
-// overlapping leaf children are handled left then right, then the walk descends into the
-// left internal child if it overlaps, and on the way back up into the right one.  Handling
-// contacts in the same order keeps the float sums identical to the reference's.
+// Traversal keeps a short stack and finds what it drops again through the tree's parent links, so
+// that no depth is too great (the reference has an int[64] stack).  The visit order is the
+// reference's (RB_BVHKernels.cu:145-214): at an internal node, its overlapping leaf children are
+// handled left then right, then the walk descends into the left internal child if it overlaps,
+// and on the way back up into the right one.  Handling contacts in the same order keeps the float
+// sums identical to the reference's.
 #include <algorithm>
 
 #include "ar_internal.cuh"
@@ -93,8 +94,8 @@ __global__ void __launch_bounds__(256) parents_kernel(int n, const int32_t* __re
 // ---- collideBVHSoARigidBody (Kernels/RB_BVHKernels.cu:100-244) ------------------------------
 __global__ void __launch_bounds__(128) collide_bvh_kernel(
     ar_sim_params prm, const int32_t* __restrict__ rb_idx, const float4* __restrict__ rel,
-    const float4* __restrict__ vel, const uint8_t* __restrict__ is_leaf,
-    const int32_t* __restrict__ left, const int32_t* __restrict__ right,
+    const float4* __restrict__ vel, const int32_t* __restrict__ left,
+    const int32_t* __restrict__ right,
     const int32_t* __restrict__ parent, const float4* __restrict__ cms,
     const float4* __restrict__ bounds, const int32_t* __restrict__ sorted_idx,
     const float* __restrict__ radii, int n, float4* __restrict__ p_force,
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(128) collide_bvh_kernel(
   float4 corr = make_float4(0.f, 0.f, 0.f, 0.f);
   const float3 r3 = ar::xyz(qrel);
   if (n >= 2) {
-    ar_lbvh::walk(n, n, is_leaf, left, right, parent,
+    ar_lbvh::walk(n, n, left, right, parent,
          [&](int c) { return c != index && overlap(qbox, load_box(bounds, c)); },
          [&](int c, bool is_left) {
            const int oc = __ldg(sorted_idx + c);
@@ -142,8 +143,8 @@ __global__ void __launch_bounds__(128) collide_bvh_kernel(
 
 // ---- FindRigidBodyCollisionsBVHKernel (Kernels/RB_BVHKernels.cu:760-876) ---------------------
 __global__ void __launch_bounds__(128) find_contacts_kernel(
-    const int32_t* __restrict__ rb_idx, const uint8_t* __restrict__ is_leaf,
-    const int32_t* __restrict__ left, const int32_t* __restrict__ right,
+    const int32_t* __restrict__ rb_idx, const int32_t* __restrict__ left,
+    const int32_t* __restrict__ right,
     const int32_t* __restrict__ parent, const int32_t* __restrict__ max_r,
     const float4* __restrict__ cms, const float4* __restrict__ bounds,
     const int32_t* __restrict__ sorted_idx, const float* __restrict__ radii, int n,
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(128) find_contacts_kernel(
   float best = contact_distance[q];
   int best_p = 0, best_b = 0;
   bool found = false;
-  ar_lbvh::walk(n, n, is_leaf, left, right, parent,
+  ar_lbvh::walk(n, n, left, right, parent,
        [&](int c) {
          return c != index && __ldg(max_r + c) >= index && overlap(qbox, load_box(bounds, c));
        },
@@ -187,8 +188,8 @@ __global__ void __launch_bounds__(128) find_contacts_kernel(
 
 // ---- contact pairs through the BVH ------------------------------------------------------------
 __global__ void __launch_bounds__(128) pairs_bvh_kernel(
-    float two_r, const int32_t* __restrict__ rb_idx, const uint8_t* __restrict__ is_leaf,
-    const int32_t* __restrict__ left, const int32_t* __restrict__ right,
+    float two_r, const int32_t* __restrict__ rb_idx, const int32_t* __restrict__ left,
+    const int32_t* __restrict__ right,
     const int32_t* __restrict__ parent, const float4* __restrict__ cms,
     const float4* __restrict__ bounds, const int32_t* __restrict__ sorted_idx, int n,
     int2* __restrict__ pairs, int capacity, int* __restrict__ count, int* __restrict__ err) {
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(128) pairs_bvh_kernel(
   const float4 qpos = __ldg(cms + index);
   const Box qbox = load_box(bounds, index);
   const int qbody = __ldg(rb_idx + q);
-  ar_lbvh::walk(n, n, is_leaf, left, right, parent,
+  ar_lbvh::walk(n, n, left, right, parent,
        [&](int c) { return c != index && overlap(qbox, load_box(bounds, c)); },
        [&](int c, bool) {
          if (c < index) return;  // each unordered pair once (from its lower sorted leaf)
@@ -236,8 +237,8 @@ __device__ __forceinline__ bool sphere_box(float4 p, const Box& b, float r) {
 // be NULL): green when a leaf is within touching distance.
 __global__ void __launch_bounds__(128) collide_bvh_static_kernel(
     ar_sim_params prm, const int32_t* __restrict__ rb_idx, const float4* __restrict__ rel,
-    const float4* __restrict__ pos, float4* __restrict__ vel, const uint8_t* __restrict__ is_leaf,
-    const int32_t* __restrict__ left, const int32_t* __restrict__ right,
+    const float4* __restrict__ pos, float4* __restrict__ vel, const int32_t* __restrict__ left,
+    const int32_t* __restrict__ right,
     const int32_t* __restrict__ parent, const float4* __restrict__ cms,
     const float4* __restrict__ bounds, const float* __restrict__ radii, int m, int n,
     float4* __restrict__ p_force, float4* __restrict__ p_torque, float4* __restrict__ color) {
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(128) collide_bvh_static_kernel(
     const float3 r3 = ar::xyz(__ldg(rel + i));
     float3 force = ar::mk3(0.f, 0.f, 0.f), torque = force;
     if (m >= 2) {
-      ar_lbvh::walk(m, m, is_leaf, left, right, parent,
+      ar_lbvh::walk(m, m, left, right, parent,
                     [&](int c) { return sphere_box(qpos, load_box(bounds, c), qrad); },
                     [&](int c, bool) {
                       const float4 cp = __ldg(cms + c);
@@ -284,8 +285,8 @@ __global__ void __launch_bounds__(128) collide_bvh_static_kernel(
 // the query's index; the two agree when every radius is the particle radius).  color4 (may be
 // NULL): green on a contact, white when none.
 __global__ void __launch_bounds__(128) find_bvh_static_kernel(
-    ar_sim_params prm, const float4* __restrict__ pos, const uint8_t* __restrict__ is_leaf,
-    const int32_t* __restrict__ left, const int32_t* __restrict__ right,
+    ar_sim_params prm, const float4* __restrict__ pos, const int32_t* __restrict__ left,
+    const int32_t* __restrict__ right,
     const int32_t* __restrict__ parent, const float4* __restrict__ cms,
     const float4* __restrict__ bounds, const int32_t* __restrict__ sorted_idx,
     const float* __restrict__ radii, int m, int n, float* __restrict__ contact_distance,
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(128) find_bvh_static_kernel(
     float deepest = contact_distance[i];
     int best = contact_point[i], ncol = 0;
     if (m >= 2) {
-      ar_lbvh::walk(m, m, is_leaf, left, right, parent,
+      ar_lbvh::walk(m, m, left, right, parent,
                     [&](int c) { return sphere_box(qpos, load_box(bounds, c), qrad); },
                     [&](int c, bool) {
                       const int s = __ldg(sorted_idx + c);
@@ -398,7 +399,7 @@ ar_status ar_collide_bvh_dem(ar_ctx* ctx, const ar_sim_params* params, const int
   parent = parents_or_derive(ctx, n, left, right, parent, arh::stream(stream));
   if (!parent && n >= 2) return AR_ERR_OOM;
   collide_bvh_kernel<<<arh::grid_for(n, 128), 128, 0, arh::stream(stream)>>>(
-      *params, rb_idx, (const float4*)rel4, (const float4*)vel4, is_leaf, left, right, parent,
+      *params, rb_idx, (const float4*)rel4, (const float4*)vel4, left, right, parent,
       (const float4*)cms4, (const float4*)bounds8, sorted_idx, radii, n, (float4*)p_force4,
       (float4*)p_torque4, (float4*)p_positions4);
   return arh::check_launch("ar_collide_bvh_dem");
@@ -421,7 +422,7 @@ ar_status ar_collide_bvh_static(ar_ctx* ctx, const ar_sim_params* params, const 
   if (!parent && num_scene >= 2) return AR_ERR_OOM;
   const unsigned grid = std::min(arh::grid_for(n, 128), (unsigned)ctx->num_sms * 16);
   collide_bvh_static_kernel<<<grid, 128, 0, st>>>(
-      *params, rb_idx, (const float4*)rel4, (const float4*)pos4, (float4*)vel4, is_leaf, left,
+      *params, rb_idx, (const float4*)rel4, (const float4*)pos4, (float4*)vel4, left,
       right, parent, (const float4*)cms4, (const float4*)bounds8, radii, num_scene, n,
       (float4*)p_force4, (float4*)p_torque4, (float4*)color4);
   return arh::check_launch("ar_collide_bvh_static");
@@ -446,7 +447,7 @@ ar_status ar_find_contacts_bvh_static(ar_ctx* ctx, const ar_sim_params* params,
   if (!parent && num_scene >= 2) return AR_ERR_OOM;
   const unsigned grid = std::min(arh::grid_for(n, 128), (unsigned)ctx->num_sms * 16);
   find_bvh_static_kernel<<<grid, 128, 0, st>>>(
-      *params, (const float4*)pos4, is_leaf, left, right, parent, (const float4*)cms4,
+      *params, (const float4*)pos4, left, right, parent, (const float4*)cms4,
       (const float4*)bounds8, sorted_idx, radii, num_scene, n, contact_distance, contact_point,
       (float4*)color4);
   return arh::check_launch("ar_find_contacts_bvh_static");
@@ -467,7 +468,7 @@ ar_status ar_find_contacts_bvh(ar_ctx* ctx, const int32_t* rb_idx, const uint8_t
   parent = parents_or_derive(ctx, n, left, right, parent, arh::stream(stream));
   if (!parent) return AR_ERR_OOM;
   find_contacts_kernel<<<arh::grid_for(n, 128), 128, 0, arh::stream(stream)>>>(
-      rb_idx, is_leaf, left, right, parent, max_r, (const float4*)cms4, (const float4*)bounds8,
+      rb_idx, left, right, parent, max_r, (const float4*)cms4, (const float4*)bounds8,
       sorted_idx, radii, n, contact_distance, colliding_particle, colliding_body);
   return arh::check_launch("ar_find_contacts_bvh");
 }
@@ -486,7 +487,7 @@ ar_status ar_pairs_bvh(ar_ctx* ctx, float radius, const int32_t* rb_idx, const u
   parent = parents_or_derive(ctx, n, left, right, parent, st);
   if (!parent) return AR_ERR_OOM;
   pairs_bvh_kernel<<<arh::grid_for(n, 128), 128, 0, st>>>(
-      2.0f * radius, rb_idx, is_leaf, left, right, parent, (const float4*)cms4,
+      2.0f * radius, rb_idx, left, right, parent, (const float4*)cms4,
       (const float4*)bounds8, sorted_idx, n, (int2*)pairs2, capacity, d_count, ctx->d_err);
   return arh::check_launch("ar_pairs_bvh");
 }

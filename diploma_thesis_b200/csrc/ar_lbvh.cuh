@@ -160,42 +160,61 @@ __device__ __forceinline__ bool overlap(const Box& a, const Box& b) {
          (a.lz <= b.hz && a.hz >= b.lz);
 }
 
-// ---- stackless traversal in the reference's order (RB_BVHKernels.cu:145-214) -------------------
+// ---- traversal in the reference's order (RB_BVHKernels.cu:145-214) ------------------------------
 // From internal node `root`: at each internal node, the overlapping leaf children are handled
 // left then right, then the walk descends into the left internal child if it overlaps, and on
 // the way back up into the right one.  visit_leaf(leaf, is_left_child) for every leaf child
-// that accept(child) admits.  `root` is never left through its parent link.  A valid tree is
-// walked in fewer than 4 (2n - 1) moves; the bound only guards against a malformed tree.
+// that accept(child) admits (leaves are the nodes below n).  `root` is never left through its
+// parent link.
+//
+// The right children to come back to wait on a short stack, the newest kStack of them: a tree
+// over 32-bit keys rarely needs more.  Older ones are dropped, and found again once the stack is
+// empty by climbing the parent links from the subtree just finished, so that no depth is too
+// great.  Climbing after every subtree instead reads each node's links and boxes a second time on
+// the way up (132,651 packed particles: 341 -> 175 us).  A valid tree is walked in fewer than 4 (2n - 1) moves; the bound only
+// guards against a malformed tree.
+constexpr int kStack = 32;  // a power of two
 template <class Accept, class Visit>
-__device__ __forceinline__ void walk(int root, int n, const uint8_t* __restrict__ is_leaf,
-                                     const int32_t* __restrict__ left,
+__device__ __forceinline__ void walk(int root, int n, const int32_t* __restrict__ left,
                                      const int32_t* __restrict__ right,
                                      const int32_t* __restrict__ parent, Accept accept,
                                      Visit visit_leaf) {
-  int node = root;
-  bool descending = true;
-  int from = -1;
+  int stack[kStack];
+  int top = 0, bottom = 0;  // entries bottom .. top - 1, at their index mod kStack
+  int node = root, start = root;  // start: the root of the subtree being walked
   for (long moves = 8l * n + 64; moves > 0; --moves) {
-    if (descending) {
-      const int lc = __ldg(left + node), rc = __ldg(right + node);
-      const bool ll = __ldg(is_leaf + lc), rl = __ldg(is_leaf + rc);
-      const bool ol = accept(lc), orr = accept(rc);
-      if (ol && ll) visit_leaf(lc, true);
-      if (orr && rl) visit_leaf(rc, false);
-      if (ol && !ll) { node = lc; continue; }
-      if (orr && !rl) { node = rc; continue; }
-      descending = false;
-    } else {
-      const int rc = __ldg(right + node);
-      if (from == __ldg(left + node) && !__ldg(is_leaf + rc) && accept(rc)) {
-        node = rc;
-        descending = true;
-        continue;
+    const int lc = __ldg(left + node), rc = __ldg(right + node);
+    const bool ol = accept(lc), orr = accept(rc);
+    if (ol && lc < n) visit_leaf(lc, true);
+    if (orr && rc < n) visit_leaf(rc, false);
+    const bool tl = ol && lc >= n, tr = orr && rc >= n;
+    if (tl) {
+      if (tr) {
+        stack[top++ & (kStack - 1)] = rc;
+        if (top - bottom > kStack) ++bottom;
       }
+      node = lc;
+      continue;
     }
-    if (node == root) return;
-    from = node;
-    node = __ldg(parent + node);
+    if (tr) {
+      node = rc;
+      continue;
+    }
+    if (top > bottom) {
+      node = start = stack[--top & (kStack - 1)];
+      continue;
+    }
+    if (bottom == 0) return;  // nothing was dropped
+    // climb from the finished subtree to the next right child that was dropped
+    for (node = start; moves > 0; --moves) {
+      if (node == root) return;
+      const int up = __ldg(parent + node), r = __ldg(right + up);
+      if (node != r && r >= n && accept(r)) {
+        node = start = r;
+        break;
+      }
+      node = up;
+    }
   }
 }
 

@@ -400,7 +400,8 @@ __device__ __forceinline__ uint32_t near_cell(const SceneDev& S, uint32_t local,
 // load the cells' entries, a prefix sum over their counts numbers the candidates in cell order,
 // each lane tests one, and the contacts' forces are added in that order with a partial sum per
 // cell.  One thread per particle waits out a dependent round trip per row and candidate with too
-// few warps to hide it (@FEW@).
+// few warps to hide it (1,728 packed particles: 22.5 ->
+// 6 us; the rule stands at kFewPerSm).
 template <bool kOne>
 __global__ void __launch_bounds__(256) collide_few_kernel(
     const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table, int nt, int per_warp,
@@ -763,6 +764,13 @@ __global__ void __launch_bounds__(ar_tree::kTile, 6) bvh_tree_kernel(
   ar_tree::build_up(s, &box, m, n, lcp, out, work);
 }
 
+// Half of a wide node in one 32-byte load.
+__device__ __forceinline__ void load_half_node(const float4* p, float4* a, float4* b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a->x), "=f"(a->y), "=f"(a->z), "=f"(a->w), "=f"(b->x), "=f"(b->y), "=f"(b->z),
+        "=f"(b->w) : "l"(p));
+}
+
 // DEM gather through the scene's subtree in the reference's visit order
 // (collideBVHSoARigidBody, Kernels/RB_BVHKernels.cu:145-214): at a node the overlapping leaf
 // children are handled left then right, then the walk goes into the left internal child if it
@@ -809,8 +817,9 @@ __global__ void __launch_bounds__(256) bvh_collide_kernel(
     int top = 0;
     int node = root;
     for (int guard = 2 * nt; guard > 0; --guard) {
-      const float4* c = nodes[node - nt].c;
-      const float4 a0 = __ldg(c), a1 = __ldg(c + 1), b0 = __ldg(c + 2), b1 = __ldg(c + 3);
+      float4 a0, a1, b0, b1;
+      load_half_node(nodes[node - nt].c, &a0, &a1);
+      load_half_node(nodes[node - nt].c + 2, &b0, &b1);
       const int lc = __float_as_int(a1.z), rc = __float_as_int(b1.z);
       // a child holding only this particle's body (this particle's own leaf included) is skipped
       const bool ol = __float_as_int(a1.w) != body &&

@@ -49,8 +49,8 @@ __device__ __forceinline__ float3 gnormalize(float3 v) {
 
 // ---- FindRigidBodyCollisionsUniformGridKernel (Kernels/RB_UniformGridKernels.cu:731-842) --------
 // Per sorted particle: over the 27 neighbour cells (z, y, x = -1..1), occupants of other bodies;
-// the deepest penetration 2r - |p - q| above the running maximum (re-read per cell, as the
-// reference does) is kept with the other particle's original index and body.
+// the deepest penetration 2r - |p - q| above the running maximum is kept with the other particle's
+// original index and body.
 __global__ void __launch_bounds__(128) find_contacts_grid_kernel(
     ar_grid::Grid g, float radius, const int32_t* __restrict__ rb_idx,
     const float4* __restrict__ spos, const uint32_t* __restrict__ gidx,
@@ -64,28 +64,30 @@ __global__ void __launch_bounds__(128) find_contacts_grid_kernel(
   const uint32_t orig = __ldg(gidx + index);
   const int body = __ldg(rb_idx + orig);
   const float threshold = 2 * radius;
-  for (int z = -1; z <= 1; ++z)
-    for (int y = -1; y <= 1; ++y)
-      for (int x = -1; x <= 1; ++x) {
-        const uint32_t h = g.hash(make_int3(gp.x + x, gp.y + y, gp.z + z));
-        const uint32_t st = __ldg(cstart + h);
-        float best = contact_distance[orig];
-        if (st == ar::kEmpty) continue;
-        const uint32_t en = __ldg(cend + h);
-        for (uint32_t j = st; j < en; ++j) {
-          const int o2 = (int)__ldg(gidx + j);
-          const int b2 = __ldg(rb_idx + o2);
-          if (j == (uint32_t)index || b2 == body) continue;
-          const float3 d = sub3(pos, f3(__ldg(spos + j)));
-          const float dist = sqrtf(ar::dot(d, d));
-          if (threshold - dist > best) {
-            best = threshold - dist;
-            contact_distance[orig] = best;
-            colliding_particle[orig] = o2;
-            colliding_body[orig] = b2;
-          }
-        }
-      }
+  const float reach2_up = nextafterf(threshold * threshold, INFINITY);
+  float best = contact_distance[orig];
+  int best_particle = -1, best_body = 0;
+  ar_grid::for_occupied(g, gp, cstart, cend, [&](uint32_t st, uint32_t en) {
+    for (uint32_t j = st; j < en; ++j) {
+      const float3 d = sub3(pos, f3(__ldg(spos + j)));
+      const float d2 = ar::dot(d, d);
+      // from the square just above threshold^2 on, the root is at least the threshold
+      if (best >= 0.f && !(d2 < reach2_up)) continue;
+      const float depth = threshold - sqrtf(d2);
+      if (!(depth > best) || j == (uint32_t)index) continue;
+      const int o2 = (int)__ldg(gidx + j);
+      const int b2 = __ldg(rb_idx + o2);
+      if (b2 == body) continue;
+      best = depth;
+      best_particle = o2;
+      best_body = b2;
+    }
+  });
+  if (best_particle >= 0) {
+    contact_distance[orig] = best;
+    colliding_particle[orig] = best_particle;
+    colliding_body[orig] = best_body;
+  }
 }
 
 // ---- GatherRigidBodyCollisions (Particles/updateFunctions.cpp:1431-1500) -----------------------
@@ -285,100 +287,222 @@ __global__ void __launch_bounds__(256) sis_geometry_kernel(
   }
 }
 
-// A contact in the solver's working order: 11 float4 words -- normal and bias, the four
-// geometry words, the two masses and body ids, the two inverse inertias -- stored word-major
-// (word k of contact p at k * stride + p), so that a warp loading consecutive contacts reads
-// each word as one contiguous run.
-constexpr int kRecWords = 11;
-__device__ __forceinline__ void pack_contact(const Contacts& C, const Bodies& B,
-                                             const Geometry* __restrict__ geo, int c,
-                                             float4* __restrict__ out, size_t stride) {
+// x / d for the solver's divisors, which do not change from sweep to sweep, from r = 1 / d: two
+// residual corrections of x * r.  The first leaves an error well below one unit in the last place,
+// and then the second one's result is the correctly rounded quotient, since r is the correctly
+// rounded reciprocal and the residual is exact (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990).  Holds for |x| and d in the ranges tested below, in
+// which nothing over- or underflows; a zero dividend gives the zero of IEEE division's sign.
+__device__ __forceinline__ float div_by(float x, float d, float r) {
+  const float q0 = x * r;
+  const float q1 = fmaf(fmaf(-q0, d, x), r, q0);
+  const float q2 = fmaf(fmaf(-q1, d, x), r, q1);
+  return copysignf(q2, q0);
+}
+__device__ __forceinline__ bool div_dividend(float x) {  // zero, or 2^-70 <= |x| < 2^60
+  const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+  return u - 0x1c800000u < 0x5d800000u - 0x1c800000u || u == 0;
+}
+__device__ __forceinline__ bool div_divisor(float d) {  // 2^-40 <= |d| < 2^40
+  const uint32_t u = __float_as_uint(d) & 0x7fffffffu;
+  return u - 0x2b800000u < 0x53800000u - 0x2b800000u;
+}
+
+// A contact in the solver's working order: two halves, one per body, solved by two neighbouring
+// lanes.  A half is five float4 words, stored in blocks of 32 halves, word by word, so that a warp
+// loading consecutive contacts reads each word as one or two contiguous runs (half h of the packed
+// order at half_at(h), its words 32 apart; the halves of contact p are 2 p and 2 p + 1):
+//   normal, bias | lever arm, mc | inverse inertia 0..3 | 4..7 |
+//   inverse inertia 8, mass, 1 / mass, body and flags
+// The second half's inverse inertia, mass and 1 / mass are negated: its body takes the opposite
+// impulse, and negated factors give exactly the negated products, sums and quotients.
+// A contact with one body has no second half; its place holds what the first one's friction needs:
+//   t1, k1 | t2, k2 | - | - | friction bound, -, -, flags
+// Beside them two floats per half that change: the impulse and the number of sweeps done (first
+// half); 1 / mc, or a one-body contact's two frictions (second half).
+constexpr int kHalfWords = 5;
+constexpr uint32_t kOneBody = 1u << 31, kSelfPair = 1u << 30, kBodyMask = kSelfPair - 1;  // flags
+__device__ __forceinline__ size_t half_at(int h) {
+  return (size_t)(h >> 5) * (32 * kHalfWords) + (h & 31);
+}
+// Returns whether the contact needs the general form of solve_half.
+__device__ __forceinline__ bool pack_contact(const Contacts& C, const Bodies& B,
+                                             const Geometry* __restrict__ geo, int c, int p,
+                                             float4* __restrict__ rec,
+                                             float2* __restrict__ accs) {
   const int i1 = C.body1[c], i2 = C.body2[c];
   const float4 n = C.normal[c];
   const Geometry g = geo[c];
-  float I1[9], I2[9];
+  const uint32_t flags = i2 < 0 ? kOneBody : (i2 == i1 ? kSelfPair : 0u);
+  bool general = flags != 0u || !div_divisor(g.g0.w);
+  auto half = [&](int side, float4 arm, int body) {
+    const float sign = side ? -1.f : 1.f, m = sign * B.mass[body];
+    float I[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    I1[k] = B.inv_inertia[9 * i1 + k];
-    I2[k] = i2 >= 0 ? B.inv_inertia[9 * i2 + k] : 0.f;
+    for (int k = 0; k < 9; ++k) I[k] = sign * B.inv_inertia[9 * body + k];
+    float4* out = rec + half_at(2 * p + side);
+    out[0] = make_float4(n.x, n.y, n.z, C.bias[c]);
+    out[32] = make_float4(arm.x, arm.y, arm.z, g.g0.w);
+    out[64] = make_float4(I[0], I[1], I[2], I[3]);
+    out[96] = make_float4(I[4], I[5], I[6], I[7]);
+    out[128] = make_float4(I[8], m, 1.0f / m, __uint_as_float((uint32_t)body | flags));
+    general |= !div_divisor(m);
+  };
+  half(0, g.g0, i1);
+  if (i2 >= 0) {
+    half(1, g.g1, i2);
+  } else {
+    float4* out = rec + half_at(2 * p + 1);
+    out[0] = g.g2;
+    out[32] = g.g3;
+    out[128] = make_float4(g.g1.w, 0.f, 0.f, __uint_as_float(flags));
   }
-  out[0 * stride] = make_float4(n.x, n.y, n.z, C.bias[c]);
-  out[1 * stride] = g.g0;
-  out[2 * stride] = g.g1;
-  out[3 * stride] = g.g2;
-  out[4 * stride] = g.g3;
-  out[5 * stride] = make_float4(B.mass[i1], i2 >= 0 ? B.mass[i2] : 1.f, __int_as_float(i1),
-                       __int_as_float(i2));
-  out[6 * stride] = make_float4(I1[0], I1[1], I1[2], I1[3]);
-  out[7 * stride] = make_float4(I1[4], I1[5], I1[6], I1[7]);
-  out[8 * stride] = make_float4(I1[8], I2[0], I2[1], I2[2]);
-  out[9 * stride] = make_float4(I2[3], I2[4], I2[5], I2[6]);
-  out[10 * stride] = make_float4(I2[7], I2[8], 0.f, 0.f);
+  accs[2 * (size_t)p] = make_float2(C.acc_impulse[c], __int_as_float(0));
+  accs[2 * (size_t)p + 1] = i2 >= 0 ? make_float2(1.0f / g.g0.w, 0.f)
+                                    : make_float2(C.acc_friction[c], C.acc_friction2[c]);
+  return general;
 }
 
-// One contact's update: the velocity-dependent part of the reference's loop body.  acc holds
-// the accumulated impulse and the two accumulated frictions.
-__device__ void solve_packed(const float4* r, float4* acc, const Bodies& B,
-                             float upper_bound) {
-  const float3 n = f3(r[0]);
-  const float bias = r[0].w;
-  const float3 p1 = f3(r[1]), t1 = f3(r[3]), t2 = f3(r[4]);
-  const float mc = r[1].w, bound = r[2].w, k1 = r[3].w, k2 = r[4].w;
-  const float m1 = r[5].x, m2 = r[5].y;
-  const int i1 = __float_as_int(r[5].z), i2 = __float_as_int(r[5].w);
-  const float I1[9] = {r[6].x, r[6].y, r[6].z, r[6].w, r[7].x, r[7].y, r[7].z, r[7].w, r[8].x};
-  const float4 a = *acc;
-  float3 v1 = f3(B.vel[i1]), w1 = f3(B.ang[i1]);
-  if (i2 == -1) {
-    const float3 vel = add3(v1, cross3(w1, p1));
-    const float v_rel = dot3(vel, n);
-    float corrective = qdiv(-(v_rel + bias), mc);
-    const float tmp = clampf(a.x + corrective, 0.f, upper_bound);
-    corrective = tmp - a.x;
-    float cf1 = qdiv(-dot3(vel, t1), k1);
-    const float f1 = clampf(a.y + cf1, -bound, bound);
-    cf1 = f1 - a.y;
-    float cf2 = qdiv(-dot3(vel, t2), k2);
-    const float f2 = clampf(a.z + cf2, -bound, bound);
-    cf2 = f2 - a.z;
-    *acc = make_float4(tmp, f1, f2, 0.f);
-    const float3 imp = add3(add3(mul3(corrective, n), mul3(cf1, t1)), mul3(cf2, t2));
-    v1 = add3(v1, qdiv3(imp, m1));
-    w1 = add3(w1, mv(I1, cross3(p1, imp)));
-    B.vel[i1] = make_float4(v1.x, v1.y, v1.z, 0.f);
-    B.ang[i1] = make_float4(w1.x, w1.y, w1.z, 0.f);
-    return;
-  }
-  const float3 p2 = f3(r[2]);
-  const float I2[9] = {r[8].y, r[8].z, r[8].w, r[9].x, r[9].y, r[9].z, r[9].w, r[10].x, r[10].y};
-  float3 v2 = f3(B.vel[i2]), w2 = f3(B.ang[i2]);
-  const float v_rel = dot3(add3(v1, cross3(w1, p1)), n) - dot3(add3(v2, cross3(w2, p2)), n);
-  float corrective = qdiv(-(v_rel + bias), mc);
-  const float tmp = clampf(a.x + corrective, 0.f, upper_bound);
-  corrective = tmp - a.x;
-  // friction is accumulated as the reference does, but (as there) not applied between bodies
-  const float3 vel = add3(add3(add3(mul3(-1.f, v1), cross3(w1, p1)), v2), cross3(w2, p2));
-  *acc = make_float4(tmp, clampf(a.y + qdiv(-dot3(vel, t1), k1), -bound, bound),
-                     clampf(a.z + qdiv(-dot3(vel, t2), k2), -bound, bound), 0.f);
-  const float3 imp = mul3(corrective, n);
-  v1 = add3(v1, qdiv3(imp, m1));
-  w1 = add3(w1, mv(I1, cross3(p1, imp)));
-  B.vel[i1] = make_float4(v1.x, v1.y, v1.z, 0.f);
-  B.ang[i1] = make_float4(w1.x, w1.y, w1.z, 0.f);
-  v2 = sub3(v2, qdiv3(imp, m2));
-  w2 = sub3(w2, mv(I2, cross3(p2, imp)));
-  B.vel[i2] = make_float4(v2.x, v2.y, v2.z, 0.f);
-  B.ang[i2] = make_float4(w2.x, w2.y, w2.z, 0.f);
+// Half of a contact, held in registers (h: its place, -1: none).
+struct Half {
+  float4 w[kHalfWords];
+  float2 acc;
+  int h;
+};
+// Loads from L2 at this point of the program: the compiler would move plain loads down to their
+// uses, a step later, to save registers.
+__device__ __forceinline__ float4 load_now(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 load_now(const float2* p) {
+  float2 v;
+  asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void load_half(const float4* rec, const float2* accs, int h, Half& it) {
+  it.h = h;
+  if (h < 0) return;
+  const float4* at = rec + half_at(h);
+#pragma unroll
+  for (int k = 0; k < kHalfWords; ++k) it.w[k] = load_now(at + 32 * k);
+  it.acc = load_now(accs + h);
 }
 
-constexpr int kSisThreads = 320;   // the sweep block
-constexpr int kLevelCap = 8192;    // level runs kept in shared memory up to this many levels
+// One contact's update, the velocity-dependent part of the reference's loop body, by the two
+// lanes that hold its halves (every lane of the warp calls it).  Each lane takes its body's share
+// of the relative velocity, both compute the impulse, and each updates its body.  Friction between
+// two bodies is accumulated but never applied (as in the reference), so only the relative velocity
+// it needs is kept, in `vrel`, for sis_friction_kernel.  kGeneral: some contact of the list has one
+// body, or one body twice, or a divisor outside div_by's range.
+// What an update leaves to be stored: no other update waits for it, so it is done in the next
+// step, between that step's dependent operations.
+struct Rest {
+  int h = -1, sweep;
+  float total;
+  float3 v, c;  // the body's velocity before the update, and angular velocity x lever arm
+};
+// The accumulated impulse, and the relative velocity for the friction as the reference sums it.
+__device__ __forceinline__ void store_rest(const Rest& r, float2* __restrict__ accs,
+                                           float4* __restrict__ vrel, size_t stride) {
+  auto pair = [&](float x) { return __shfl_xor_sync(0xffffffffu, x, 1); };
+  const float3 v2 = ar::mk3(pair(r.v.x), pair(r.v.y), pair(r.v.z));
+  const float3 c2 = ar::mk3(pair(r.c.x), pair(r.c.y), pair(r.c.z));
+  const float3 slide = add3(add3(add3(mul3(-1.f, r.v), r.c), v2), c2);
+  if (r.h >= 0 && !(threadIdx.x & 1)) {
+    accs[r.h] = make_float2(r.total, __int_as_float(r.sweep + 1));
+    vrel[(size_t)r.sweep * stride + (r.h >> 1)] = make_float4(slide.x, slide.y, slide.z, 0.f);
+  }
+}
+template <bool kGeneral>
+__device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ accs, float4* vel,
+                                           float4* ang, float4* __restrict__ vrel, size_t stride,
+                                           float upper_bound, Rest& rest) {
+  constexpr uint32_t kAll = 0xffffffffu;
+  const bool side = threadIdx.x & 1;
+  const bool have = it.h >= 0;
+  const uint32_t tag = have ? __float_as_uint(it.w[4].w) : 0u;
+  const bool one = kGeneral && (tag & kOneBody);
+  const bool mine = have && !(one && side);  // this lane holds a body
+  const int body = mine ? (int)(tag & kBodyMask) : 0;
+  const float3 n = f3(it.w[0]), arm = f3(it.w[1]);
+  const float mc = it.w[1].w, m = it.w[4].y;
+  const float3 v = f3(vel[body]), w = f3(ang[body]);
+  store_rest(rest, accs, vrel, stride);  // the previous update's
+  // the first lane's impulse against the second one's 1 / mc
+  const float met = __shfl_xor_sync(kAll, it.acc.x, 1);
+  const float acc = side ? met : it.acc.x;
+  const float3 c = cross3(w, arm);
+  const float3 at = add3(v, c);  // the body's velocity at the contact
+  const float s = dot3(at, n);
+  const float d = s - __shfl_xor_sync(kAll, s, 1);
+  const float v_rel = one ? s : (side ? -d : d);
+  const float x = -(v_rel + it.w[0].w);
+  float change;
+  if (kGeneral) {
+    change = qdiv(x, mc);
+  } else {
+    change = div_by(x, mc, side ? it.acc.x : met);
+    if (!div_dividend(x)) change = x / mc;
+  }
+  const float total = clampf(acc + change, 0.f, upper_bound);
+  float3 imp = mul3(total - acc, n);
+  if (kGeneral && __any_sync(kAll, one)) {
+    // one body: the second lane computes the frictions, which are applied
+    auto pair = [&](float3 a) {  // the other half's
+      return ar::mk3(__shfl_xor_sync(kAll, a.x, 1), __shfl_xor_sync(kAll, a.y, 1),
+                     __shfl_xor_sync(kAll, a.z, 1));
+    };
+    const float3 vel1 = pair(at);
+    float cf1 = 0.f, cf2 = 0.f;
+    if (one && side) {
+      const float bound = it.w[4].x;
+      cf1 = qdiv(-dot3(vel1, f3(it.w[0])), it.w[0].w);
+      const float f1 = clampf(it.acc.x + cf1, -bound, bound);
+      cf1 = f1 - it.acc.x;
+      cf2 = qdiv(-dot3(vel1, f3(it.w[1])), it.w[1].w);
+      const float f2 = clampf(it.acc.y + cf2, -bound, bound);
+      cf2 = f2 - it.acc.y;
+      accs[it.h] = make_float2(f1, f2);
+    }
+    const float3 fx = pair(mul3(cf1, f3(it.w[0]))), fy = pair(mul3(cf2, f3(it.w[1])));
+    if (one) imp = add3(add3(imp, fx), fy);
+  }
+  float3 dv;
+  if (kGeneral) {
+    dv = qdiv3(imp, m);
+  } else {
+    const float rm = it.w[4].z;
+    dv = ar::mk3(div_by(imp.x, m, rm), div_by(imp.y, m, rm), div_by(imp.z, m, rm));
+    if (!(div_dividend(imp.x) && div_dividend(imp.y) && div_dividend(imp.z)))
+      dv = ar::mk3(imp.x / m, imp.y / m, imp.z / m);
+  }
+  const float I[9] = {it.w[2].x, it.w[2].y, it.w[2].z, it.w[2].w, it.w[3].x,
+                      it.w[3].y, it.w[3].z, it.w[3].w, it.w[4].x};
+  const float3 nv = add3(v, dv), nw = add3(w, mv(I, cross3(arm, imp)));
+  if (mine && (!kGeneral || side || !(tag & kSelfPair))) {  // a self pair: the second half stands
+    vel[body] = make_float4(nv.x, nv.y, nv.z, 0.f);
+    ang[body] = make_float4(nw.x, nw.y, nw.z, 0.f);
+  }
+  rest = Rest{it.h, __float_as_int(it.acc.y), total, v, c};
+}
+
+// Threads of the sweep block, two lanes per contact, and the bodies from which it has the larger
+// number: a step holds more contacts the more bodies there are (512 cubes: 54 at most, 4,096: 282),
+// and idle warps cost every step a little (512 cubes: 3.78 ms with 256 threads, 4.04 with 640; 27
+// cubes: 2.47 and 3.57; 3,375 cubes of 8: 3.36 ms with 640).
+constexpr int kSisFew = 256, kSisMany = 640;
+constexpr int kSisManyBodies = 1024;
+constexpr int kMaxSweeps = 32;     // sweeps per schedule (relative velocities kept for each)
 constexpr int kLevelChunk = 2048;  // body pairs staged per step of the level walk
 constexpr int kLayoutThreads = 1024;
 constexpr size_t kSisSmemMax = 220 * 1024;   // the sweep block's dynamic shared memory
 constexpr size_t kWalkSmemMax = 200 * 1024;  // the walk's (its static 16 KB stay below 227 KB)
-// The schedule's header in scratch memory: levels, shift, contact count.
-enum { kHdrLevels = 0, kHdrShift = 1, kHdrCount = 2, kHdrWords = 4 };
+// The schedule's header in scratch memory: levels, shift, contact count, and whether some contact
+// needs the general update.
+enum { kHdrLevels = 0, kHdrShift = 1, kHdrCount = 2, kHdrGeneral = 3, kHdrWords = 4 };
 
 // Schedule.  Each contact gets a level: 1 + the highest level among earlier contacts on either
 // of its bodies.  Sweep s solves level b at step b + s * shift of one schedule, where shift
@@ -474,8 +598,9 @@ __global__ void __launch_bounds__(256) sis_levels_kernel(
   __syncthreads();
   if (threadIdx.x == 0) {
     hdr[kHdrLevels] = top;
-    hdr[kHdrShift] = max(2, s_span + 1);
+    hdr[kHdrShift] = max(4, s_span + 1);
     hdr[kHdrCount] = count;
+    hdr[kHdrGeneral] = 0;
   }
 }
 
@@ -550,139 +675,155 @@ __global__ void __launch_bounds__(kLayoutThreads) sis_layout_kernel(const int* _
 __global__ void __launch_bounds__(256) sis_pack_kernel(Contacts C, Bodies B,
                                                        const Geometry* __restrict__ geo,
                                                        const int* __restrict__ level,
-                                                       const int* __restrict__ hdr,
-                                                       int capacity, int2* __restrict__ run,
+                                                       int* __restrict__ hdr,
+                                                       int2* __restrict__ run,
                                                        int* __restrict__ order,
                                                        float4* __restrict__ rec,
-                                                       float4* __restrict__ accs) {
+                                                       float2* __restrict__ accs) {
   const int count = hdr[kHdrCount];
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < count; c += gridDim.x * blockDim.x) {
     const int p = atomicAdd(&run[level[c]].x, 1);
     order[p] = c;
-    pack_contact(C, B, geo, c, rec + p, (size_t)capacity);
-    accs[p] = make_float4(C.acc_impulse[c], C.acc_friction[c], C.acc_friction2[c], 0.f);
+    if (pack_contact(C, B, geo, c, p, rec, accs)) hdr[kHdrGeneral] = 1;
   }
 }
 
-// The accumulated impulses back to the caller's arrays, in contact order.
-__global__ void __launch_bounds__(256) sis_writeback_kernel(Contacts C,
-                                                            const int* __restrict__ hdr,
-                                                            const int* __restrict__ order,
-                                                            const float4* __restrict__ accs) {
+// After a schedule of `sweeps` sweeps: the accumulated impulses back to the caller's arrays, and
+// the frictions of the contacts between two bodies, sweep by sweep from the relative velocities
+// that the sweeps kept (the reference accumulates them in its loop; nothing else reads them).
+// The sweep counts start again at zero for the next schedule.
+__global__ void __launch_bounds__(256) sis_friction_kernel(Contacts C,
+                                                           const Geometry* __restrict__ geo,
+                                                           const int* __restrict__ hdr,
+                                                           const int* __restrict__ order,
+                                                           const float4* __restrict__ vrel,
+                                                           size_t stride, int sweeps,
+                                                           float2* __restrict__ accs) {
   const int count = hdr[kHdrCount];
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
     const int c = order[p];
-    const float4 a = accs[p];
-    C.acc_impulse[c] = a.x;
-    C.acc_friction[c] = a.y;
-    C.acc_friction2[c] = a.z;
+    const float impulse = accs[2 * (size_t)p].x;
+    C.acc_impulse[c] = impulse;
+    accs[2 * (size_t)p] = make_float2(impulse, __int_as_float(0));
+    if (C.body2[c] < 0) {
+      const float2 f = accs[2 * (size_t)p + 1];
+      C.acc_friction[c] = f.x;
+      C.acc_friction2[c] = f.y;
+      continue;
+    }
+    const float bound = geo[c].g1.w;
+    const float4 t1 = geo[c].g2, t2 = geo[c].g3;
+    float f1 = C.acc_friction[c], f2 = C.acc_friction2[c];
+    for (int s = 0; s < sweeps; ++s) {
+      const float3 v = f3(__ldcg(vrel + s * stride + p));
+      f1 = clampf(f1 + qdiv(-dot3(v, f3(t1)), t1.w), -bound, bound);
+      f2 = clampf(f2 + qdiv(-dot3(v, f3(t2)), t2.w), -bound, bound);
+    }
+    C.acc_friction[c] = f1;
+    C.acc_friction2[c] = f2;
   }
 }
 
-// A packed contact and its accumulators, held in registers.
-struct Item {
-  float4 r[kRecWords];
-  float4 acc;
-  int p;  // packed index, -1: none
-};
-
-__device__ __forceinline__ void load_item(const float4* rec, size_t stride, const float4* accs,
-                                          int p, Item& it) {
-  it.p = p;
-  if (p < 0) return;
-#pragma unroll
-  for (int k = 0; k < kRecWords; ++k) it.r[k] = __ldcg(rec + k * stride + p);
-  it.acc = __ldcg(accs + p);
+// The contacts of one step of the schedule, [lo, hi): the levels b congruent to the step (mod
+// shift) with max(1, step - (sweeps - 1) shift) <= b <= min(levels, step).
+__device__ __forceinline__ int2 step_range(int step, int levels, int sweeps, int shift,
+                                           const int2* runs) {
+  if (step > levels + (sweeps - 1) * shift) return make_int2(0, 0);
+  const int most = min(step, levels), least = max(1, step - (sweeps - 1) * shift);
+  const int hi = most - (most - step % shift + shift) % shift;  // largest such level
+  const int lo = least + (step - least) % shift;                // smallest
+  return lo <= hi && hi >= 1 ? make_int2(runs[lo].y, runs[hi].x) : make_int2(0, 0);
 }
 
-// The per-sweep levels lo, lo + shift, ..., hi that one step of the schedule covers, advanced
-// one step at a time without division.
-struct StepRange {
-  int lo, hi;  // the step has contacts while lo <= hi
-  int step;
-  __device__ void advance(int levels, int iterations, int shift) {
-    ++step;
-    // the largest level <= min(step, levels) congruent to step
-    if (++hi > levels) hi -= shift;
-    // the smallest level >= max(1, step - (iterations - 1) shift) congruent to step
-    if (step - 1 < iterations * shift) {
-      if (++lo > shift) lo -= shift;
-    } else {
-      ++lo;
+// The steps of a schedule of `sweeps` sweeps, in order, with a barrier between them.  Each lane
+// loads its half of a contact two steps ahead (record and accumulators, from L2), into the
+// registers of the one it has just solved: its accumulators were last written one step after the
+// last update, shift >= 4 steps before they are needed, so their writer has passed a barrier since.
+template <bool kGeneral, int kThreads>
+__device__ __forceinline__ void run_schedule(int levels, int shift, int capacity, int sweeps,
+                                             float upper_bound, const int2* runs,
+                                             const float4* rec, float2* accs, float4* vel,
+                                             float4* ang, float4* vrel, int2* s_range) {
+  const int steps = levels + (sweeps - 1) * shift;  // fits in int: checked by the host
+  constexpr int kTable = (kThreads - 2) / 2 * 2;    // steps per table, two more looked up
+  const int lane = threadIdx.x;  // this lane's half in a step's first round
+  Rest rest;
+  rest.v = rest.c = ar::mk3(0.f, 0.f, 0.f);
+  auto fetch = [&](int2 r, Half& it) {
+    load_half(rec, accs, 2 * r.x + lane < 2 * r.y ? 2 * r.x + lane : -1, it);
+  };
+  auto solve = [&](Half& it, int2 r, int2 ahead) {
+    if (__any_sync(0xffffffffu, it.h >= 0 || rest.h >= 0)) {
+      solve_half<kGeneral>(it, accs, vel, ang, vrel, capacity, upper_bound, rest);
+      for (int h0 = 2 * r.x + kThreads; h0 < 2 * r.y; h0 += kThreads) {
+        // contacts beyond one per lane pair
+        load_half(rec, accs, h0 + lane < 2 * r.y ? h0 + lane : -1, it);
+        solve_half<kGeneral>(it, accs, vel, ang, vrel, capacity, upper_bound, rest);
+      }
+    }
+    fetch(ahead, it);
+    __syncthreads();
+  };
+  Half a, b;
+  for (int base = 1; base <= steps; base += kTable) {
+    s_range[threadIdx.x] = step_range(base + (int)threadIdx.x, levels, sweeps, shift, runs);
+    __syncthreads();
+    if (base == 1) {
+      fetch(s_range[0], a);
+      fetch(s_range[1], b);
+    }
+    const int count = min(kTable, steps - base + 1);
+    // two buffers in turn (a register move would wait for the loads in flight); kTable is even, so
+    // every table starts with the same buffer
+    for (int i = 0; i < count; i += 2) {
+      solve(a, s_range[i], s_range[i + 2]);
+      if (i + 1 >= count) break;
+      solve(b, s_range[i + 1], s_range[i + 3]);
     }
   }
-};
+  store_rest(rest, accs, vrel, capacity);
+}
 
-// The sweeps, in one block: the steps are solved in order with a barrier between them; each
-// thread loads its item of the next step (record and accumulators, from L2) while it solves
-// the current one, which is safe because an item's accumulators were last written
-// shift >= 2 steps earlier.  kShared: the bodies' velocities and angular velocities live in
-// shared memory.
-template <bool kShared>
-__global__ void __launch_bounds__(kSisThreads) sis_sweep_kernel(
-    Bodies B, const int* __restrict__ hdr, int capacity, int num_bodies, int iterations,
+// The sweeps, in one block.  kShared: the bodies' velocities and angular velocities live in shared
+// memory.
+// Bound by the serial chain of steps and by issue on one SM: 7,966 steps of up to 282 contacts on
+// 4,096 packed cubes, 0.93 us each, of which a contact's dependent operations, a barrier and 190
+// instructions per warp.  13.7 -> 7.4 ms against a lane per contact with divisions (510
+// instructions), its friction and its accumulators before the barrier, and loads one step ahead
+// that the step did not cover.  Tried: a cluster of two or four blocks, each with all velocities
+// and storing into the others' (a cluster barrier per step costs 0.7 us: 13 ms); copying the first
+// words to shared memory two steps ahead with cp.async (fewer stalls, a quarter more
+// instructions: 9.7 ms); three register buffers (spills: 28 ms).
+template <bool kShared, int kThreads>
+__global__ void __launch_bounds__(kThreads) sis_sweep_kernel(
+    Bodies B, const int* __restrict__ hdr, int capacity, int num_bodies, int sweeps,
     float upper_bound, const int2* __restrict__ run, const float4* __restrict__ rec,
-    float4* __restrict__ accs) {
-  // (kShared) vel[num_bodies], ang[num_bodies], then the level runs when they fit
-  extern __shared__ float4 s_mem[];
+    float2* __restrict__ accs, float4* __restrict__ vrel) {
+  extern __shared__ float4 s_bodies[];  // (kShared) vel[num_bodies], ang[num_bodies]
+  __shared__ int2 s_range[kThreads];
   const int levels = hdr[kHdrLevels], shift = hdr[kHdrShift];
-  float4* s_bodies = s_mem;
-  int2* s_run = reinterpret_cast<int2*>(s_bodies + (kShared ? 2 * num_bodies : 0));
-  Bodies W = B;
-  const int2* runs = run;
-  if (levels + 1 <= kLevelCap) {
-    for (int l = threadIdx.x; l <= levels; l += blockDim.x) s_run[l] = run[l];
-    runs = s_run;
-  }
+  float4 *vel = B.vel, *ang = B.ang;
   if (kShared) {
+    vel = s_bodies;
+    ang = s_bodies + num_bodies;
     for (int b = threadIdx.x; b < num_bodies; b += blockDim.x) {
-      s_bodies[b] = B.vel[b];
-      s_bodies[num_bodies + b] = B.ang[b];
+      vel[b] = B.vel[b];
+      ang[b] = B.ang[b];
     }
-    W.vel = s_bodies;
-    W.ang = s_bodies + num_bodies;
   }
   __syncthreads();
   if (levels > 0) {
-    const int steps = levels + (iterations - 1) * shift;  // fits in int: checked by the host
-    StepRange nr{1, 1, 1};  // step 1 covers level 1 of sweep 0 only
-    int next_lo = runs[1].y, next_hi = runs[1].x;
-    Item nxt;
-    load_item(rec, capacity, accs,
-              next_lo + (int)threadIdx.x < next_hi ? next_lo + (int)threadIdx.x : -1, nxt);
-    for (int step = 1; step <= steps; ++step) {
-      const Item cur = nxt;
-      const int lo = next_lo, hi = next_hi;
-      if (step < steps) {
-        nr.advance(levels, iterations, shift);
-        next_lo = next_hi = 0;
-        if (nr.lo <= nr.hi) {
-          next_lo = runs[nr.lo].y;
-          next_hi = runs[nr.hi].x;
-        }
-        const int p = next_lo + (int)threadIdx.x;
-        load_item(rec, capacity, accs, p < next_hi ? p : -1, nxt);
-      }
-      if (cur.p >= 0) {
-        float4 a = cur.acc;
-        solve_packed(cur.r, &a, W, upper_bound);
-        accs[cur.p] = a;
-        // items beyond one per thread
-        for (int p = lo + (int)(threadIdx.x + blockDim.x); p < hi; p += blockDim.x) {
-          Item more;
-          load_item(rec, capacity, accs, p, more);
-          a = more.acc;
-          solve_packed(more.r, &a, W, upper_bound);
-          accs[p] = a;
-        }
-      }
-      __syncthreads();
-    }
+    if (hdr[kHdrGeneral])
+      run_schedule<true, kThreads>(levels, shift, capacity, sweeps, upper_bound, run, rec, accs,
+                                   vel, ang, vrel, s_range);
+    else
+      run_schedule<false, kThreads>(levels, shift, capacity, sweeps, upper_bound, run, rec, accs,
+                                    vel, ang, vrel, s_range);
   }
   if (kShared) {
     for (int b = threadIdx.x; b < num_bodies; b += blockDim.x) {
-      B.vel[b] = W.vel[b];
-      B.ang[b] = W.ang[b];
+      B.vel[b] = vel[b];
+      B.ang[b] = ang[b];
     }
   }
 }
@@ -765,20 +906,26 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
     arh::set_error("iterations x (capacity + 1) must stay below 2^31");
     return AR_ERR_INVALID_ARG;
   }
-  // scratch: geometry[capacity] (64-byte aligned), records (word-major) and accumulators,
-  // level runs run[capacity + 1], the schedule header, then level[capacity], order[capacity],
-  // last[num_bodies], first[num_bodies]
-  const size_t geo_bytes = sizeof(Geometry) * (size_t)capacity;
-  const size_t rec_bytes = sizeof(float4) * (size_t)capacity * (kRecWords + 1);
-  const size_t run_bytes = sizeof(int2) * ((size_t)capacity + 1);
-  const size_t words = kHdrWords + 2 * (size_t)capacity + 2 * (size_t)num_bodies;
-  char* base = (char*)arh::scratch(ctx, geo_bytes + rec_bytes + run_bytes + sizeof(int) * words);
+  // scratch: geometry[capacity] (64-byte aligned), the halves' records (word-major), the relative
+  // velocities of a schedule's sweeps, the accumulators, level runs run[capacity + 1], the
+  // schedule header, then level[capacity], order[capacity], last[num_bodies], first[num_bodies]
+  const int batch = std::min(iterations, kMaxSweeps);
+  const size_t cap = (size_t)capacity;
+  const size_t geo_bytes = sizeof(Geometry) * cap;
+  const size_t rec_bytes = sizeof(float4) * ((2 * cap + 31) / 32 * 32) * kHalfWords;
+  const size_t vrel_bytes = sizeof(float4) * cap * batch;
+  const size_t acc_bytes = sizeof(float2) * 2 * cap;
+  const size_t run_bytes = sizeof(int2) * (cap + 1);
+  const size_t words = kHdrWords + 2 * cap + 2 * (size_t)num_bodies;
+  char* base = (char*)arh::scratch(ctx, geo_bytes + rec_bytes + vrel_bytes + acc_bytes +
+                                            run_bytes + sizeof(int) * words);
   if (!base) return AR_ERR_OOM;
   Geometry* geo = (Geometry*)base;
   float4* rec = (float4*)(base + geo_bytes);
-  float4* accs = rec + (size_t)capacity * kRecWords;
-  int2* run = (int2*)(base + geo_bytes + rec_bytes);
-  int* hdr = (int*)(base + geo_bytes + rec_bytes + run_bytes);
+  float4* vrel = (float4*)((char*)rec + rec_bytes);
+  float2* accs = (float2*)(vrel + cap * batch);
+  int2* run = (int2*)(accs + 2 * cap);
+  int* hdr = (int*)(run + cap + 1);
   int* level = hdr + kHdrWords;
   int* order = level + capacity;
   int* last = order + capacity;
@@ -805,23 +952,22 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
   }
   sis_sizes_kernel<<<gg, 256, 0, st>>>(level, hdr, run);
   sis_layout_kernel<<<1, kLayoutThreads, 0, st>>>(hdr, run, order);
-  sis_pack_kernel<<<gg, 256, 0, st>>>(C, B, geo, level, hdr, capacity, run, order, rec, accs);
-  // sweeps: level runs in shared memory; the bodies' velocities too when they fit
-  const size_t base_smem = sizeof(int2) * (size_t)kLevelCap;
-  const size_t smem = base_smem + 32 * (size_t)num_bodies;
-  if (smem <= kSisSmemMax) {
-    cudaFuncSetAttribute(sis_sweep_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    sis_sweep_kernel<true><<<1, kSisThreads, smem, st>>>(B, hdr, capacity, num_bodies,
-                                                         iterations, 100.f, run, rec, accs);
-  } else {
-    cudaFuncSetAttribute(sis_sweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)base_smem);
-    sis_sweep_kernel<false><<<1, kSisThreads, base_smem, st>>>(B, hdr, capacity, num_bodies,
-                                                               iterations, 100.f, run, rec,
-                                                               accs);
+  sis_pack_kernel<<<gg, 256, 0, st>>>(C, B, geo, level, hdr, run, order, rec, accs);
+  // sweeps: the bodies' velocities in shared memory when they fit; more threads for scenes with
+  // many contacts per step
+  const size_t body_smem = 32 * (size_t)num_bodies;
+  const bool shared = body_smem <= kSisSmemMax;
+  const size_t smem = shared ? body_smem : 0;
+  const bool many = num_bodies >= kSisManyBodies;
+  auto* sweep = !shared ? sis_sweep_kernel<false, kSisMany>
+                        : (many ? sis_sweep_kernel<true, kSisMany> : sis_sweep_kernel<true, kSisFew>);
+  cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  for (int done = 0; done < iterations; done += batch) {
+    const int sweeps = std::min(batch, iterations - done);
+    sweep<<<1, !shared || many ? kSisMany : kSisFew, smem, st>>>(
+        B, hdr, capacity, num_bodies, sweeps, 100.f, run, rec, accs, vrel);
+    sis_friction_kernel<<<gg, 256, 0, st>>>(C, geo, hdr, order, vrel, cap, sweeps, accs);
   }
-  sis_writeback_kernel<<<gg, 256, 0, st>>>(C, hdr, order, accs);
   return arh::check_launch("ar_sequential_impulse");
 }
 

@@ -58,24 +58,123 @@ __global__ void __launch_bounds__(256) leaves_kernel(int n, const int32_t* __res
 }
 
 // ---- refit (kernelConstructInternalNodesSoA, BVHSoAKernels.cu:148-176) ----------------------
+// One thread per leaf climbs (ar_lbvh::refit_climb): the better form while the launch, and not the
+// number of arrivals, bounds it.
 __global__ void __launch_bounds__(256) refit_kernel(int n, const int32_t* __restrict__ left,
                                                     const int32_t* __restrict__ right,
                                                     const int32_t* __restrict__ parent,
-                                                    float4* bounds, int* __restrict__ counters) {
+                                                    float4* bounds, int* counters) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  auto children = [&](int node, ar_lbvh::Box6* a, ar_lbvh::Box6* b) {
-    const int l = __ldg(left + node), r = __ldg(right + node);
-    const float4 a0 = __ldcg(bounds + 2 * l), a1 = __ldcg(bounds + 2 * l + 1);
-    const float4 b0 = __ldcg(bounds + 2 * r), b1 = __ldcg(bounds + 2 * r + 1);
-    *a = ar_lbvh::Box6{a0.x, a0.y, a0.z, a0.w, a1.x, a1.y};
-    *b = ar_lbvh::Box6{b0.x, b0.y, b0.z, b0.w, b1.x, b1.y};
+  if (i < n) ar_lbvh::refit_climb(i, n, left, right, parent, bounds, counters);
+}
+
+// From this many leaves on the tiles below pay for their second launch (both forms: 300,000 points
+// 47.7 us alone, 59.1 in tiles; 600,000: 69.6, 71.7; 1,000,003: 92.5, 89.1; 2,000,000: 151, 126;
+// with a climb that read both boxes and the links one after another: 57, 82, 110, 183).
+constexpr int kRefitTilesFrom = 1 << 20;
+// A block takes kRefitTile consecutive leaves and the internal nodes of the same numbers.  The
+// subtrees that lie within these are merged in shared memory, the second child to arrive at a node
+// merging both.  The largest of them are left to refit_open_kernel, which climbs the rest of the
+// tree through global memory with ar_lbvh::refit_climb: a block that climbed on by itself would
+// keep its place on the SM for its longest climb (2^24 points: 1006 us, without the prefetched
+// links).  Any tree is refitted;
+// Karras' numbering, which gives a node the number of one end of its leaves, makes all but about
+// one node in twenty-five merge in shared memory, where a climb of every leaf through device-scope
+// arrivals was bound by these (2^24 points: 953 -> 691 us).
+// A subtree left over is named in the counter of a merged node, which nothing arrives at, as
+// -(its root + 1); a tile with more of them than merged nodes climbs from the rest itself.
+constexpr int kRefitTile = 256;
+__global__ void __launch_bounds__(kRefitTile) refit_tiles_kernel(int n, const int32_t* __restrict__ left,
+                                                           const int32_t* __restrict__ right,
+                                                           const int32_t* __restrict__ parent,
+                                                           float4* bounds,
+                                                           int* __restrict__ counters) {
+  constexpr int kT = kRefitTile;
+  __shared__ float4 s_a[2 * kT], s_b[2 * kT];  // boxes: the tile's leaves, then its nodes
+  __shared__ short s_child[2][kT];             // places of a node's children, -1: elsewhere
+  __shared__ short s_parent[2 * kT];           // node of the tile above a place, -1: elsewhere
+  __shared__ int s_met[kT];                    // children that have arrived
+  __shared__ short s_slot[kT];                 // the merged nodes
+  __shared__ int s_slots, s_open;
+  const int t = threadIdx.x, base = blockIdx.x * kT, k = base + t;
+  auto place = [&](int c) {
+    const unsigned leaf = (unsigned)(c - base), node = (unsigned)(c - n - base);
+    if (c < n) return leaf < (unsigned)kT ? (int)leaf : -1;
+    return node < (unsigned)kT ? kT + (int)node : -1;
   };
-  auto store = [&](int node, const ar_lbvh::Box6& m) {
-    __stcg(bounds + 2 * node, make_float4(m.lx, m.ly, m.lz, m.hx));
-    __stcg(bounds + 2 * node + 1, make_float4(m.hy, m.hz, 0.f, 0.f));
+  if (k < n) {
+    s_a[t] = __ldcs(bounds + 2 * k);
+    s_b[t] = __ldcs(bounds + 2 * k + 1);
+  }
+  int lc = -1, rc = -1;
+  if (k < n - 1) {
+    lc = place(__ldg(left + n + k));
+    rc = place(__ldg(right + n + k));
+  }
+  s_child[0][t] = (short)lc;
+  s_child[1][t] = (short)rc;
+  s_parent[t] = s_parent[kT + t] = -1;
+  s_met[t] = 0;
+  if (t == 0) s_slots = s_open = 0;
+  __syncthreads();
+  if (lc >= 0 && rc >= 0) s_parent[lc] = s_parent[rc] = (short)t;
+  __syncthreads();
+  if (k < n) {
+    int c = t, p = s_parent[t];
+    float4 a = s_a[t], b = s_b[t];
+    for (int guard = 0; guard < kT && p >= 0; ++guard, p = s_parent[c]) {
+      __threadfence_block();  // this child's box before its arrival
+      if (atomicAdd(&s_met[p], 1) != 1) break;
+      __threadfence_block();  // its sibling's box after that one's arrival
+      const bool is_left = s_child[0][p] == c;
+      const int o = s_child[is_left ? 1 : 0][p];
+      const float4 oa = s_a[o], ob = s_b[o];
+      const ar_lbvh::Box6 u = is_left ? ar_lbvh::merge_boxes(ar_lbvh::box6(a, b), ar_lbvh::box6(oa, ob))
+                                      : ar_lbvh::merge_boxes(ar_lbvh::box6(oa, ob), ar_lbvh::box6(a, b));
+      c = kT + p;
+      a = s_a[c] = make_float4(u.lx, u.ly, u.lz, u.hx);
+      b = s_b[c] = make_float4(u.hy, u.hz, 0.f, 0.f);
+    }
+  }
+  __syncthreads();
+  // the merged nodes' boxes; the leaves and merged nodes whose parent is not merged are left over
+  const bool merged = s_met[t] >= 2;
+  if (merged) {
+    __stcg(bounds + 2 * (size_t)(n + k), s_a[kT + t]);
+    __stcg(bounds + 2 * (size_t)(n + k) + 1, s_b[kT + t]);
+  }
+  auto open = [&](int c) { return s_parent[c] < 0 || s_met[s_parent[c]] < 2; };
+  const bool open_leaf = k < n && open(t), open_node = merged && open(kT + t);
+  if (merged) s_slot[atomicAdd(&s_slots, 1)] = (short)t;
+  const int at = open_leaf || open_node ? atomicAdd(&s_open, (int)open_leaf + (int)open_node) : 0;
+  __syncthreads();
+  auto leave = [&](int root, int i) {
+    if (i < s_slots) counters[base + s_slot[i]] = -(root + 1);
+    else ar_lbvh::refit_climb(root, n, left, right, parent, bounds, counters);
   };
-  ar_lbvh::refit_climb(i, n, parent, counters, children, store);
+  if (open_leaf) leave(k, at);
+  if (open_node) leave(n + k, at + (int)open_leaf);
+}
+
+// The climb from the subtrees that refit_kernel left over: a block collects those of kRefitScan
+// counters, so that its threads climb together.
+constexpr int kRefitScan = 4096;
+__global__ void __launch_bounds__(256) refit_open_kernel(int n, const int32_t* __restrict__ left,
+                                                         const int32_t* __restrict__ right,
+                                                         const int32_t* __restrict__ parent,
+                                                         float4* bounds, int* counters) {
+  __shared__ int s_root[kRefitScan];
+  __shared__ int s_count;
+  if (threadIdx.x == 0) s_count = 0;
+  __syncthreads();
+  const long base = (long)blockIdx.x * kRefitScan;
+  for (int i = threadIdx.x; i < kRefitScan; i += blockDim.x) {
+    const int v = base + i < n - 1 ? __ldcg(counters + base + i) : 0;
+    if (v < 0) s_root[atomicAdd(&s_count, 1)] = -v - 1;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < s_count; i += blockDim.x)
+    ar_lbvh::refit_climb(s_root[i], n, left, right, parent, bounds, counters);
 }
 
 // Parent links from the child links, for callers with the reference's traversal signature
@@ -380,8 +479,15 @@ ar_status ar_lbvh_refit(ar_ctx* ctx, int n, const int32_t* left, const int32_t* 
   if (!counters) return AR_ERR_OOM;
   cudaStream_t st = arh::stream(stream);
   cudaMemsetAsync(counters, 0, (size_t)(n - 1) * sizeof(int), st);
-  refit_kernel<<<arh::grid_for(n, 256), 256, 0, st>>>(n, left, right, parent, (float4*)bounds8,
-                                                      counters);
+  if (n < kRefitTilesFrom) {
+    refit_kernel<<<arh::grid_for(n, 256), 256, 0, st>>>(n, left, right, parent, (float4*)bounds8,
+                                                        counters);
+  } else {
+    refit_tiles_kernel<<<arh::grid_for(n, kRefitTile), kRefitTile, 0, st>>>(
+        n, left, right, parent, (float4*)bounds8, counters);
+    refit_open_kernel<<<arh::grid_for(n - 1, kRefitScan), 256, 0, st>>>(
+        n, left, right, parent, (float4*)bounds8, counters);
+  }
   return arh::check_launch("ar_lbvh_refit");
 }
 

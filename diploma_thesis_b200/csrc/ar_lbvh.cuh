@@ -106,13 +106,11 @@ __device__ __forceinline__ int2 karras_node(int i, int n, const Lcp& lcp, uint8_
 }
 
 // ---- bottom-up refit (kernelConstructInternalNodesSoA, BVHSoAKernels.cu:148-176) ------------
-// One thread per leaf climbs; the second thread to reach a node merges its children's boxes
-// (mergeBounds, BVHAuxiliary.cuh:83-94: min of the mins and max of the maxes, left child
-// first) and continues.  The arrival counter is a device-scope acquire-release increment, so
-// the first thread's box stores (made before its increment) are visible to the second
-// thread's loads (made after it); boxes are read and written through L2.  (Merging the nodes
-// inside a block through shared memory instead was measured slower: more dependent loads per
-// level outweighed the fences it saved.)
+// The second thread to reach a node merges its children's boxes (mergeBounds,
+// BVHAuxiliary.cuh:83-94: min of the mins and max of the maxes, left child first) and climbs on.
+// The arrival counter is a device-scope acquire-release increment, so the first thread's box
+// stores (made before its increment) are visible to the second thread's loads (made after it);
+// boxes are read and written through L2.
 struct Box6 {
   float lx, ly, lz, hx, hy, hz;
 };
@@ -127,22 +125,43 @@ __device__ __forceinline__ int arrive(int* counter) {
   return a.fetch_add(1, cuda::memory_order_acq_rel);
 }
 
-// Climb from `leaf`.  `children(node, &left_box, &right_box)` reads both child boxes of
-// `node` through L2; `store(node, box)` publishes a node's merged box (before the next
-// arrival).  Returns when this thread arrived first or at the root.
-template <class Children, class Store>
-__device__ __forceinline__ void refit_climb(int leaf, int n, const int32_t* __restrict__ parent,
-                                            int* __restrict__ counters, Children children,
-                                            Store store) {
-  int node = __ldg(parent + leaf);
+__device__ __forceinline__ Box6 box6(const float4& a, const float4& b) {
+  return Box6{a.x, a.y, a.z, a.w, b.x, b.y};
+}
+// Climb from `from`, a node whose box is final, merging and storing the boxes of the nodes at which
+// this thread arrives second (two float4 per node).  A level costs two dependent round trips, the
+// arrival and the sibling's box: the links of the next node are loaded with the box, and the
+// child's own box is at hand.
+__device__ __forceinline__ void refit_climb(int from, int n, const int32_t* __restrict__ left,
+                                            const int32_t* __restrict__ right,
+                                            const int32_t* __restrict__ parent, float4* bounds,
+                                            int* counters) {
+  auto inner = [&](int node) { return node >= n && node < 2 * n - 1; };  // else malformed, or no node
+  int child = from, node = __ldg(parent + from);
+  Box6 own = box6(__ldcg(bounds + 2 * (size_t)from), __ldcg(bounds + 2 * (size_t)from + 1));
+  if (!inner(node)) return;
+  int l = __ldg(left + node), r = __ldg(right + node), up = node != n ? __ldg(parent + node) : -1;
   for (int depth = 0; depth < n; ++depth) {  // a valid tree is at most n - 1 deep
-    if (node < n || node >= 2 * n - 1) return;  // malformed parent link
     if (arrive(counters + (node - n)) == 0) return;
-    Box6 a, b;
-    children(node, &a, &b);
-    store(node, merge_boxes(a, b));
-    if (node == n) return;
-    node = __ldg(parent + node);
+    const bool is_left = l == child;
+    const float4* sib = bounds + 2 * (size_t)(is_left ? r : l);
+    const float4 a = __ldcg(sib), b = __ldcg(sib + 1);
+    int nl = -1, nr = -1, nup = -1;
+    if (inner(up)) {
+      nl = __ldg(left + up);
+      nr = __ldg(right + up);
+      if (up != n) nup = __ldg(parent + up);
+    }
+    own = is_left ? merge_boxes(own, box6(a, b)) : merge_boxes(box6(a, b), own);
+    float4* to = bounds + 2 * (size_t)node;
+    __stcg(to, make_float4(own.lx, own.ly, own.lz, own.hx));
+    __stcg(to + 1, make_float4(own.hy, own.hz, 0.f, 0.f));
+    if (!inner(up)) return;
+    child = node;
+    node = up;
+    l = nl;
+    r = nr;
+    up = nup;
   }
 }
 

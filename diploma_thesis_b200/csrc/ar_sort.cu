@@ -17,6 +17,7 @@
 //     consecutive threads, so each digit run is a coalesced write.
 // Spin waits are bounded; on timeout the kernel raises kErrTimeout and finishes the pass
 // with whatever prefix it has (the result is then garbage, but nothing hangs).
+#include <algorithm>
 #include <cuda/atomic>
 #include <mutex>
 
@@ -26,11 +27,21 @@
 namespace {
 
 constexpr int kThreads = 256;  // histogram kernel
-constexpr int kItems = 16;     // keys per thread in a digit pass
-// Threads per digit-pass tile: 512 (8192-key tiles: fewer tiles, shorter look-back chains) from
-// 2^19 keys on, 256 below (more tiles to spread over the SMs).
-inline int pass_threads(long n) { return n >= (1l << 19) ? 512 : 256; }
-inline long tile_items(long n) { return (long)pass_threads(n) * kItems; }
+// Threads per digit-pass tile (9-bit digits always take 512) and keys per thread.  A tile's time is
+// the chain of its threads' items, so 8 keys per thread while there are SMs for the tiles (below
+// 2^19 keys: 30 bits, 110,592 keys 45 -> 39 us against 16), and 16 above, with 512 threads (fewer
+// tiles, shorter look-back chains: 2,097,152 keys in 92 us, 118 with 256 threads of 8).  64-bit
+// keys always take 8: two tiles of 512 threads fit an SM, where one of 16 keys filled it (63 bits,
+// 1,000,003 keys: 130 -> 120 us, 4,000,000: 469 -> 354).
+constexpr long kManyKeys = 1l << 19;
+inline int pass_threads(long n) { return n >= kManyKeys ? 512 : 256; }
+inline int pass_items(long n, size_t key_bytes) { return n >= kManyKeys && key_bytes == 4 ? 16 : 8; }
+inline long tile_items(long n, size_t key_bytes) {
+  return (long)pass_threads(n) * pass_items(n, key_bytes);
+}
+inline long tiles_for(long n, size_t key_bytes) {
+  return (n + tile_items(n, key_bytes) - 1) / tile_items(n, key_bytes);
+}
 constexpr int kRadix = ar_sort::kMaxRadix;  // histogram / status stride per pass
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
@@ -44,7 +55,8 @@ __device__ __forceinline__ uint32_t digit_of(K key, int shift, uint32_t mask) {
   return (uint32_t)(key >> shift) & mask;
 }
 
-// ---- histogram of every pass, one read of the keys -----------------------------------------
+// ---- histogram of every pass, one read of the keys, four in flight per thread ---------------
+constexpr int kHistLoads = 4;
 template <class K>
 __global__ void __launch_bounds__(kThreads) hist_kernel(const K* __restrict__ keys, int n,
                                                        ar_sort::Plan plan,
@@ -54,10 +66,17 @@ __global__ void __launch_bounds__(kThreads) hist_kernel(const K* __restrict__ ke
   const int passes = plan.passes;
   for (int i = threadIdx.x; i < passes * kRadix; i += kThreads) (&s_hist[0][0])[i] = 0;
   __syncthreads();
-  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += gridDim.x * kThreads) {
-    K k = keys[i];
-    for (int p = 0; p < passes; ++p)
-      atomicAdd(&s_hist[p][digit_of(k, plan.shift[p], (1u << plan.bits[p]) - 1)], 1u);
+  const long stride = (long)gridDim.x * kThreads;
+  for (long i = blockIdx.x * kThreads + threadIdx.x; i < n; i += stride * kHistLoads) {
+    K k[kHistLoads];
+#pragma unroll
+    for (int u = 0; u < kHistLoads; ++u) k[u] = keys[min(i + u * stride, (long)n - 1)];
+#pragma unroll
+    for (int u = 0; u < kHistLoads; ++u) {
+      if (i + u * stride >= n) break;
+      for (int p = 0; p < passes; ++p)
+        atomicAdd(&s_hist[p][digit_of(k[u], plan.shift[p], (1u << plan.bits[p]) - 1)], 1u);
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < passes * kRadix; i += kThreads) {
@@ -66,28 +85,8 @@ __global__ void __launch_bounds__(kThreads) hist_kernel(const K* __restrict__ ke
   }
 }
 
-// Exclusive scan of each pass's histogram (kRadix bins; one warp per pass).
-__global__ void hist_scan_kernel(uint32_t* __restrict__ hist, int passes) {
-  ar::pdl_wait();
-  int p = threadIdx.x >> 5;
-  if (p >= passes) return;
-  uint32_t* h = hist + p * kRadix;
-  int lane = ar::lane_id();
-  uint32_t carry = 0;
-  for (int c = 0; c < kRadix; c += 32) {
-    uint32_t v = h[c + lane], x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    h[c + lane] = carry + x - v;
-    carry += __shfl_sync(0xffffffffu, x, 31);
-  }
-}
-
 // ---- one digit pass ---------------------------------------------------------------------------
-template <class K, int kT, int kBits>
+template <class K, int kT, int kBits, int kItems>
 struct PassSmem {
   K keys[kT * kItems];
   uint32_t vals[kT * kItems];
@@ -102,11 +101,11 @@ struct PassSmem {
 // bit.  Which is faster depends on the keys: match.any wins when a warp's items hold few
 // distinct digits (cell keys of particles in input order), ballots win when they hold many
 // (Morton codes).
-template <class K, int kT, int kBits, bool kMatch = false>
-__global__ void __launch_bounds__(kT, (sizeof(K) == 4 ? 1024 : 512) / kT) onesweep_kernel(
+template <class K, int kT, int kBits, int kItems, bool kMatch = false>
+__global__ void __launch_bounds__(kT, (sizeof(K) == 4 || kItems < 16 ? 1024 : 512) / kT) onesweep_kernel(
     const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, int n, int shift, int bits,
-    const uint32_t* __restrict__ digit_base, uint32_t* __restrict__ status,
+    const uint32_t* __restrict__ digit_count, uint32_t* __restrict__ status,
     uint32_t* __restrict__ tile_counter, int* __restrict__ err, long spin_limit,
     int mute_tile0) {
   ar::pdl_wait();
@@ -115,7 +114,8 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 ? 1024 : 512) / kT) oneswe
   constexpr int kTile = kT * kItems;
   constexpr int kDigits = 1 << kBits;
   static_assert(kDigits <= kT, "one digit per thread");
-  PassSmem<K, kT, kBits>& sm = *reinterpret_cast<PassSmem<K, kT, kBits>*>(smem_raw);
+  using Smem = PassSmem<K, kT, kBits, kItems>;
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t mask = (1u << bits) - 1;
 
@@ -180,20 +180,29 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 ? 1024 : 512) / kT) oneswe
       mine.store((tile == 0 ? kFlagPrefix : kFlagAgg) | tile_count, cuda::memory_order_relaxed);
   }
 
-  // tile-local exclusive scan over digits (block scan of one value per thread)
+  // exclusive scans over the digits (one per thread) of the tile's counts and of the whole input's
+  uint32_t digit_base = 0;
   {
-    uint32_t x = tile_count;
+    const uint32_t count = d < kDigits ? __ldg(digit_count + d) : 0u;
+    uint32_t x = tile_count, y = count;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      const uint32_t xo = __shfl_up_sync(0xffffffffu, x, o), yo = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) {
+        x += xo;
+        y += yo;
+      }
     }
-    __shared__ uint32_t s_wsum[kWarps];
-    if (lane == 31) s_wsum[warp] = x;
+    __shared__ uint2 s_wsum[kWarps];
+    if (lane == 31) s_wsum[warp] = make_uint2(x, y);
     __syncthreads();
-    uint32_t add = 0;
-    for (int w = 0; w < warp; ++w) add += s_wsum[w];
-    if (d < kDigits) sm.digit_start[d] = add + x - tile_count;
+    uint2 add = make_uint2(0u, 0u);
+    for (int w = 0; w < warp; ++w) {
+      add.x += s_wsum[w].x;
+      add.y += s_wsum[w].y;
+    }
+    if (d < kDigits) sm.digit_start[d] = add.x + x - tile_count;
+    digit_base = add.y + y - count;
   }
   __syncthreads();
 
@@ -258,7 +267,7 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 ? 1024 : 512) / kT) oneswe
       cuda::atomic_ref<uint32_t, cuda::thread_scope_device> mine(status[(long)tile * kRadix + d]);
       mine.store(kFlagPrefix | ((excl + tile_count) & kValueMask), cuda::memory_order_relaxed);
     }
-    sm.gofs[d] = digit_base[d] + excl;
+    sm.gofs[d] = digit_base + excl;
   }
 
 #pragma unroll
@@ -301,7 +310,7 @@ void launch_passes(const ar_sort::Plan& plan, int n, const K* keys_in, const uin
                    K* keys_out, uint32_t* vals_out, K* tmp_keys, uint32_t* tmp_vals,
                    const uint32_t* hist, uint32_t* status, uint32_t* counters, int* err,
                    cudaStream_t st, const PassOpts& o) {
-  const long status_tiles = ((long)n + tile_items(n) - 1) / tile_items(n);
+  const long status_tiles = tiles_for(n, sizeof(K));
   const K* src_k = keys_in;
   const uint32_t* src_v = vals_in;
   for (int p = 0; p < plan.passes; ++p) {
@@ -309,22 +318,25 @@ void launch_passes(const ar_sort::Plan& plan, int n, const K* keys_in, const uin
     K* dk = to_out ? keys_out : tmp_keys;
     uint32_t* dv = to_out ? vals_out : tmp_vals;
     const int bits = plan.bits[p], shift = plan.shift[p];
-    const int kt = bits > 8 ? 512 : pass_threads(n);
-    const unsigned tiles = (unsigned)(((long)n + (long)kt * kItems - 1) / ((long)kt * kItems));
-    const uint32_t* base = hist + p * kRadix;
+    const int kt = bits > 8 ? 512 : pass_threads(n), items = pass_items(n, sizeof(K));
+    const unsigned tiles = (unsigned)(((long)n + (long)kt * items - 1) / ((long)kt * items));
+    const uint32_t* count = hist + p * kRadix;
     uint32_t* stat = status + (size_t)p * status_tiles * kRadix;
-    if (bits > 8)
-      arh::launch_pdl(onesweep_kernel<K, 512, 9>, dim3(tiles), dim3(512),
-          sizeof(PassSmem<K, 512, 9>), st, src_k, src_v, dk, dv, n, shift, bits, base, stat,
-          counters + p, err, o.spin_limit, o.mute_tile0);
-    else if (kt == 512)
-      arh::launch_pdl(o.match_rank ? onesweep_kernel<K, 512, 8, true> : onesweep_kernel<K, 512, 8>,
-          dim3(tiles), dim3(512), sizeof(PassSmem<K, 512, 8>), st, src_k, src_v, dk, dv, n, shift,
-          bits, base, stat, counters + p, err, o.spin_limit, o.mute_tile0);
-    else
-      arh::launch_pdl(o.match_rank ? onesweep_kernel<K, 256, 8, true> : onesweep_kernel<K, 256, 8>,
-          dim3(tiles), dim3(256), sizeof(PassSmem<K, 256, 8>), st, src_k, src_v, dk, dv, n, shift,
-          bits, base, stat, counters + p, err, o.spin_limit, o.mute_tile0);
+    auto pass = [&](auto* kernel, size_t smem) {
+      arh::launch_pdl(kernel, dim3(tiles), dim3(kt), smem, st, src_k, src_v, dk, dv, n, shift, bits,
+                      count, stat, counters + p, err, o.spin_limit, o.mute_tile0);
+    };
+    constexpr int kMost = sizeof(K) == 4 ? 16 : 8;  // items of the 512-thread tiles
+    if (bits > 8) {
+      if (items == 16) pass(onesweep_kernel<K, 512, 9, kMost>, sizeof(PassSmem<K, 512, 9, kMost>));
+      else pass(onesweep_kernel<K, 512, 9, 8>, sizeof(PassSmem<K, 512, 9, 8>));
+    } else if (kt == 512) {
+      pass(o.match_rank ? onesweep_kernel<K, 512, 8, kMost, true>
+                        : onesweep_kernel<K, 512, 8, kMost>, sizeof(PassSmem<K, 512, 8, kMost>));
+    } else {
+      pass(o.match_rank ? onesweep_kernel<K, 256, 8, 8, true> : onesweep_kernel<K, 256, 8, 8>,
+           sizeof(PassSmem<K, 256, 8, 8>));
+    }
     src_k = dk;
     src_v = dv;
   }
@@ -354,14 +366,13 @@ ar_status sort_impl(ar_ctx* ctx, const K* keys_in, const uint32_t* vals_in, K* k
   int* err = ctx ? ctx->d_err : nullptr;
 
   if (!external_hist) {
-    cudaMemsetAsync(base, 0, ar_sort::clear_bytes(n, passes), st);
+    cudaMemsetAsync(base, 0, ar_sort::clear_bytes(n, passes, sizeof(K)), st);
     unsigned hgrid = (unsigned)((n + kThreads * 8 - 1) / (kThreads * 8));
     unsigned cap = (unsigned)(ctx ? ctx->num_sms : 148) * 4;
     if (hgrid > cap) hgrid = cap;
     if (hgrid < 1) hgrid = 1;
     arh::launch_pdl(hist_kernel<K>, dim3(hgrid), dim3(kThreads), 0, st, keys_in, n, plan, hist);
   }
-  arh::launch_pdl(hist_scan_kernel, dim3(1), dim3(32 * ar_sort::kMaxPasses), 0, st, hist, passes);
   launch_passes<K>(plan, n, keys_in, vals_in, keys_out, vals_out, tmp_keys, tmp_vals, hist,
                    status, counters, err, st, opts);
   return arh::check_launch("radix sort");
@@ -427,33 +438,39 @@ __global__ void iota_kernel(uint32_t* v, int n) {
 }
 
 // Dynamic shared-memory opt-in of every digit-pass instantiation (current device).
-template <class K, int kT, int kBits, bool kMatch = false>
+template <class K, int kT, int kBits, int kItems, bool kMatch = false>
 cudaError_t set_pass_attribute() {
-  return cudaFuncSetAttribute(onesweep_kernel<K, kT, kBits, kMatch>,
+  return cudaFuncSetAttribute(onesweep_kernel<K, kT, kBits, kItems, kMatch>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sizeof(PassSmem<K, kT, kBits>));
+                              (int)sizeof(PassSmem<K, kT, kBits, kItems>));
+}
+template <class K>
+cudaError_t set_key_attributes() {
+  constexpr int kMost = sizeof(K) == 4 ? 16 : 8;
+  cudaError_t e = set_pass_attribute<K, 256, 8, 8>();
+  if (e == cudaSuccess) e = set_pass_attribute<K, 256, 8, 8, true>();
+  if (e == cudaSuccess) e = set_pass_attribute<K, 512, 8, kMost>();
+  if (e == cudaSuccess) e = set_pass_attribute<K, 512, 8, kMost, true>();
+  if (e == cudaSuccess) e = set_pass_attribute<K, 512, 9, 8>();
+  if (e == cudaSuccess) e = set_pass_attribute<K, 512, 9, kMost>();
+  return e;
 }
 cudaError_t set_pass_attributes() {
-  cudaError_t e = set_pass_attribute<uint32_t, 256, 8>();
-  if (e == cudaSuccess) e = set_pass_attribute<uint32_t, 512, 8>();
-  if (e == cudaSuccess) e = set_pass_attribute<uint32_t, 512, 9>();
-  if (e == cudaSuccess) e = set_pass_attribute<uint32_t, 256, 8, true>();
-  if (e == cudaSuccess) e = set_pass_attribute<uint32_t, 512, 8, true>();
-  if (e == cudaSuccess) e = set_pass_attribute<uint64_t, 256, 8>();
-  if (e == cudaSuccess) e = set_pass_attribute<uint64_t, 512, 8>();
-  if (e == cudaSuccess) e = set_pass_attribute<uint64_t, 512, 9>();
-  return e;
+  const cudaError_t e = set_key_attributes<uint32_t>();
+  return e == cudaSuccess ? set_key_attributes<uint64_t>() : e;
 }
 
 // ---- allocation-free variant -------------------------------------------------------------------
 // Workspace of the u32 sort for up to kNoAllocMaxN pairs, laid out like ar_sort::layout
 // (histograms, tile counters, look-back status for 4 passes, ping-pong keys and values).
 constexpr int kNoAllocMaxN = 1 << 20;
+// the most tiles of such a sort: 256 of 2,048 keys just below kManyKeys, 128 of 8,192 above
+constexpr int kNoAllocTiles = (int)(kManyKeys / (256 * 8));
 constexpr size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t noalloc_bytes() {
   return up256(up256(up256(up256(up256((size_t)ar_sort::kMaxPasses * kRadix * 4) +
                                        ar_sort::kMaxPasses * 4) +
-                                 (size_t)4 * (kNoAllocMaxN / (256 * kItems)) * kRadix * 4) +
+                                 (size_t)4 * kNoAllocTiles * kRadix * 4) +
                            (size_t)kNoAllocMaxN * 4) +
                (size_t)kNoAllocMaxN * 4);
 }
@@ -500,7 +517,9 @@ namespace ar_sort {
 void init() { set_pass_attributes(); }
 
 Layout layout(long n, size_t key_bytes, int passes) {
-  const long tiles = (n + tile_items(n) - 1) / tile_items(n);
+  long tiles = tiles_for(n, key_bytes);
+  // room for the most tiles of any smaller sort too, so that a workspace that fits n keys fits less
+  if (n >= kManyKeys) tiles = std::max(tiles, tiles_for(kManyKeys - 1, key_bytes));
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   Layout L;
   L.hist = 0;
@@ -535,14 +554,13 @@ ar_status sort_u64(ar_ctx* ctx, const uint64_t* keys_in, const uint32_t* vals_in
                              st, ws, ws_bytes, false);
 }
 
-size_t clear_bytes(long n, int passes) {
-  const long tiles = (n + tile_items(n) - 1) / tile_items(n);
-  Layout L = layout(n, 4, passes);
-  return L.status + (size_t)passes * tiles * kRadix * sizeof(uint32_t);
+size_t clear_bytes(long n, int passes, size_t key_bytes) {
+  return layout(n, key_bytes, passes).status +
+         (size_t)passes * tiles_for(n, key_bytes) * kRadix * sizeof(uint32_t);
 }
 
 int launches(int begin_bit, int end_bit, bool external_hist) {
-  return (external_hist ? 1 : 3) + make_plan(begin_bit, end_bit).passes;
+  return (external_hist ? 0 : 2) + make_plan(begin_bit, end_bit).passes;
 }
 
 }  // namespace ar_sort
@@ -638,7 +656,6 @@ ar_status ar_radix_sort_pairs_u32_noalloc(const uint32_t* keys_in, const uint32_
   if (hgrid < 1) hgrid = 1;
   arh::launch_pdl(hist_kernel<uint32_t>, dim3(hgrid), dim3(kThreads), 0, st, keys_in, n, plan,
       hist);
-  arh::launch_pdl(hist_scan_kernel, dim3(1), dim3(32 * ar_sort::kMaxPasses), 0, st, hist, passes);
   launch_passes<uint32_t>(plan, n, keys_in, vals_in, keys_out, vals_out, tmp_keys, tmp_vals, hist,
                           status, counters, (int*)d_status, st, PassOpts());
   return arh::check_launch("allocation-free sort");

@@ -66,7 +66,7 @@ ar_status sort_u64(ar_ctx* ctx, const uint64_t* keys_in, const uint32_t* vals_in
 
 // Bytes at the head of the workspace that must be zero before a sort whose histogram is
 // accumulated externally (histograms, tile counters, look-back status).
-size_t clear_bytes(long n, int passes);
+size_t clear_bytes(long n, int passes, size_t key_bytes = 4);
 
 // Histogram of `key` for every pass of `plan` into a shared [kMaxPasses][kMaxRadix] block
 // histogram (then hist_flush), with one shared-memory atomic per distinct digit per warp (the

@@ -15,8 +15,8 @@
 //                   buckets' ranges, and the tile's header for place_kernel; every block scans
 //                   the bucket counts and the tile counts it needs itself.
 //   bucket_sort_kernel  each bucket sorted by (key, index): one warp per bucket, ranks by
-//                   comparison (in registers up to 32 movers, in shared memory up to 256, in
-//                   global memory beyond; buckets usually hold a few movers).
+//                   comparison (buckets usually hold a few movers); larger buckets by the whole
+//                   block, split by further key bits first.
 //   place_kernel    over the previous order.  A stayer (a particle that kept its key) at old
 //                   position j has r = j - (movers before j) stayers before it in the new
 //                   order too (their keys did not change and the old order is sorted), and A =
@@ -317,46 +317,107 @@ __global__ void __launch_bounds__(kThreads) bucket_kernel(const uint32_t* __rest
 }
 
 // ---- each bucket sorted by (key, index) into w.movers --------------------------------------
-// One warp per bucket; a mover's rank is the number of the bucket's movers with a smaller (key,
-// index) (they are distinct).  Up to 32 movers: one per lane, compared through shuffles; up to
-// kWarpStage: staged in the warp's shared memory and compared there; beyond: compared in
-// global memory.  (Sorting chunks of 32 and merging them by binary searches was measured
-// slower for the buckets of the 2M-particle pile, at most ~130 movers.)
-constexpr int kWarpStage = 256;
+// One warp per bucket of up to kWarpStage movers; a mover's rank is the number of the bucket's
+// movers with a smaller (key, index) (they are distinct).  Up to 32 movers: one per lane,
+// compared through shuffles; beyond: staged in the warp's shared memory and compared there.
+// (Sorting chunks of 32 and merging them by binary searches was measured slower there.)
+// Larger buckets are sorted by the whole block, one after another: the movers are first split
+// by the next kSubLog2 bits of their keys, then ranked among those of their own part.  They
+// come in bunches (the front of a falling pile, the first step after the bodies were set anew),
+// so neighbouring buckets belong to different blocks.  With a warp for every bucket the kernel was
+// bound by the quadratic count of the fullest one (2M-particle pile after an upload: Morton
+// buckets 73 -> 8.8 us, grid buckets 22 -> 7.5 us; a limit of 64 movers per warp measured the
+// same, 192 1 % of a step slower).
+constexpr int kWarpStage = 96;
+constexpr int kBlockStage = 2048;  // movers the block stages in shared memory; beyond, in global
+constexpr int kSubLog2 = 8;
+static_assert(1 << kSubLog2 == kThreads, "one part per thread in the scan");
+__device__ __forceinline__ uint2 split(unsigned long long c) {
+  return make_uint2((uint32_t)(c >> 32), (uint32_t)c);
+}
+// grid: ceil(nb / kWarps) blocks
 __global__ void __launch_bounds__(kThreads) bucket_sort_kernel(Work w) {
   ar::pdl_wait();
-  __shared__ unsigned long long s_stage[kWarps][kWarpStage];
-  const int lane = ar::lane_id();
-  unsigned long long* stage = s_stage[threadIdx.x >> 5];
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < w.nb; b += warps) {
-    const uint32_t lo = __ldg(w.bstart + b), s = __ldg(w.bstart + b + 1) - lo;
-    if (s == 0) continue;
-    const uint2* __restrict__ g = w.grouped + lo;
-    if (s <= 32) {
-      const uint2 e = lane < (int)s ? g[lane] : make_uint2(0xffffffffu, 0xffffffffu);
-      const unsigned long long ce = composite(e);
+  static_assert(kWarps * kWarpStage <= kBlockStage, "the warps share the block's stage");
+  __shared__ unsigned long long s_stage[kBlockStage];
+  __shared__ uint32_t s_part[kThreads + 1], s_fill[kThreads], s_warp[kWarps];
+  __shared__ uint2 s_big[kWarps];  // first slot and movers of each warp's bucket if it is large
+  const int lane = ar::lane_id(), warp = threadIdx.x >> 5;
+  const int b = warp * gridDim.x + blockIdx.x;
+  const uint32_t lo = b < w.nb ? __ldg(w.bstart + b) : 0u;
+  const uint32_t s = b < w.nb ? __ldg(w.bstart + b + 1) - lo : 0u;
+  const bool big = s > (uint32_t)kWarpStage;
+  if (lane == 0) s_big[warp] = make_uint2(lo, big ? s : 0u);
+  const uint2* __restrict__ g = w.grouped + lo;
+  if (s <= 32) {
+    const uint2 e = lane < (int)s ? g[lane] : make_uint2(0xffffffffu, 0xffffffffu);
+    const unsigned long long ce = composite(e);
+    uint32_t rank = 0;
+    for (uint32_t t = 0; t < s; ++t) rank += __shfl_sync(0xffffffffu, ce, t) < ce;
+    if (lane < (int)s) w.movers[lo + rank] = e;
+  } else if (!big) {
+    unsigned long long* stage = s_stage + warp * kWarpStage;
+    for (uint32_t i = lane; i < s; i += 32) stage[i] = composite(g[i]);
+    __syncwarp();
+    for (uint32_t i = lane; i < s; i += 32) {
+      const unsigned long long ce = stage[i];
       uint32_t rank = 0;
-      for (uint32_t t = 0; t < s; ++t) rank += __shfl_sync(0xffffffffu, ce, t) < ce;
-      if (lane < (int)s) w.movers[lo + rank] = e;
-    } else if (s <= (uint32_t)kWarpStage) {
-      for (uint32_t i = lane; i < s; i += 32) stage[i] = composite(g[i]);
-      __syncwarp();
-      for (uint32_t i = lane; i < s; i += 32) {
-        const unsigned long long ce = stage[i];
-        uint32_t rank = 0;
-        for (uint32_t t = 0; t < s; ++t) rank += stage[t] < ce;
-        w.movers[lo + rank] = make_uint2((uint32_t)(ce >> 32), (uint32_t)ce);
+      for (uint32_t t = 0; t < s; ++t) rank += stage[t] < ce;
+      w.movers[lo + rank] = split(ce);
+    }
+  }
+  if (!__syncthreads_or(big)) return;
+  const int sub = max(w.bshift - kSubLog2, 0);
+  const uint32_t rest = (1u << w.bshift) - 1u;  // the key's bits below the bucket's
+  for (int q = 0; q < kWarps; ++q) {
+    const uint32_t first = s_big[q].x, count = s_big[q].y;
+    if (count == 0) continue;  // the same for the whole block
+    uint2* in = w.grouped + first;
+    uint2* out = w.movers + first;
+    const bool staged = count <= (uint32_t)kBlockStage;
+    s_fill[threadIdx.x] = 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < count; i += kThreads)
+      atomicAdd(s_fill + ((in[i].x & rest) >> sub), 1u);
+    __syncthreads();
+    const uint32_t c = s_fill[threadIdx.x];
+    uint32_t incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    for (int v = 0; v < warp; ++v) incl += s_warp[v];
+    s_part[threadIdx.x + 1] = incl;
+    s_fill[threadIdx.x] = incl - c;
+    if (threadIdx.x == 0) s_part[0] = 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < count; i += kThreads) {
+      const uint2 e = in[i];
+      const uint32_t at = atomicAdd(s_fill + ((e.x & rest) >> sub), 1u);
+      if (staged) s_stage[at] = composite(e);
+      else out[at] = e;
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < count; i += kThreads) {
+      const unsigned long long ce = staged ? s_stage[i] : composite(out[i]);
+      const uint32_t d = ((uint32_t)(ce >> 32) & rest) >> sub;
+      const uint32_t from = s_part[d], to = s_part[d + 1];
+      uint32_t rank = from;
+      if (staged) {
+        for (uint32_t t = from; t < to; ++t) rank += s_stage[t] < ce;
+        out[rank] = split(ce);
+      } else {  // back into the input's place, which is read no more
+        for (uint32_t t = from; t < to; ++t) rank += composite(out[t]) < ce;
+        in[rank] = split(ce);
       }
-      __syncwarp();
-    } else {
-      for (uint32_t i = lane; i < s; i += 32) {
-        const uint2 e = g[i];
-        const unsigned long long ce = composite(e);
-        uint32_t rank = 0;
-        for (uint32_t t = 0; t < s; ++t) rank += composite(g[t]) < ce;
-        w.movers[lo + rank] = e;
-      }
+    }
+    __syncthreads();
+    if (!staged) {
+      for (uint32_t i = threadIdx.x; i < count; i += kThreads) out[i] = in[i];
+      // s_fill and s_part are not read here; the next bucket's first barrier follows
     }
   }
 }

@@ -23,17 +23,127 @@ using ar_lbvh::overlap;
 namespace {
 
 // ---- Karras 2012 internal nodes (kernelConstructRadixTreeSoA, BVHSoAKernels.cu:7-99) -------
+// Over sorted codes the common prefix of two leaves is the smallest of those of the neighbours
+// between them.  A tile of kBuildTile nodes puts the prefixes of its neighbours into shared memory
+// with their minima over 2^k of them, a byte each, and both of a node's searches (the end of its
+// range, then its split) descend through the levels: kBuildLevels steps in shared memory for every
+// lane, against as many steps, to global memory, as the warp's longest range takes in the search
+// over the codes.  The nodes whose range leaves the tile (at most one per bit of the codes and
+// side), and those that unsorted codes give equal neighbours, are gathered and search the codes
+// with eight lanes each.  Bound by issued instructions (2^24 points, 30 / 63-bit codes: 399 / 478
+// -> 242 / 255 us, 1,000,003: 36 / 42 -> 26 / 28 us; one lane for each gathered node 318 / 339 us,
+// tiles of 512 277 / 294 us, the second search from its range's own level 262 / 275 us).
+constexpr int kBuildTile = 1024;
+constexpr int kBuildThreads = 256;
+constexpr int kBuildLevels = 11;  // 2^0 to 2^10 neighbours
+// Entry q is the prefix of leaves q - 2 and q - 1 of the tile, plus one, so that 0, where there
+// are no leaves, ends every search; entries 0 and kBuildEnd, outside the tile, are 0 too.
+constexpr int kBuildEnd = kBuildTile + 2;
+constexpr int kBuildRow = kBuildEnd / 4 + 1;  // in words of four entries
+static_assert(kBuildTile + 1 < 1 << kBuildLevels, "the descent needs each level once");
 template <class Lcp>
-__global__ void __launch_bounds__(256) build_kernel(Lcp lcp, int n, uint8_t* __restrict__ is_leaf,
-                                                    int32_t* __restrict__ left,
-                                                    int32_t* __restrict__ right,
-                                                    int32_t* __restrict__ parent,
-                                                    int32_t* __restrict__ min_r,
-                                                    int32_t* __restrict__ max_r) {
+__global__ void __launch_bounds__(kBuildThreads) build_kernel(Lcp lcp, int n, ar_lbvh::TreeOut out) {
+  __shared__ uint32_t s_words[kBuildLevels][kBuildRow];
+  __shared__ uint16_t s_list[kBuildTile];
+  __shared__ int s_count;
+  const int t0 = blockIdx.x * kBuildTile;
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    out.parent[n] = -1;  // root: no parent (the reference leaves it unset)
+  if (threadIdx.x == 0) s_count = 0;
+  uint8_t* base = reinterpret_cast<uint8_t*>(s_words[0]);
+  for (int q = threadIdx.x; q < 4 * kBuildRow; q += kBuildThreads) {
+    const int k = t0 - 2 + q;
+    base[q] = (uint8_t)(q == 0 || q >= kBuildEnd || k < 0 ? 0 : lcp(k, k + 1) + 1);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int lv = 1; lv < kBuildLevels; ++lv) {
+    const int half = 1 << (lv - 1);
+    for (int w = threadIdx.x; w < kBuildRow; w += kBuildThreads) {
+      const uint32_t a = s_words[lv - 1][w];
+      const int o = w + (half < 4 ? 1 : half / 4);
+      uint32_t b = o < kBuildRow ? s_words[lv - 1][o] : 0u;
+      if (half < 4) b = __funnelshift_r(a, b, 8 * half);
+      s_words[lv][w] = __vminu4(a, b);
+    }
+    __syncthreads();
+  }
+  auto least = [&](int lv, int q) -> int {  // over the entries q .. q + 2^lv - 1
+    return base[lv * 4 * kBuildRow + q];
+  };
+  for (int u = 0; u < kBuildTile / kBuildThreads; ++u) {
+    const int q = u * kBuildThreads + threadIdx.x, i = t0 + q;
+    if (i >= n - 1) break;
+    const int before = least(0, q + 1), after = least(0, q + 2);
+    const int d = after > before ? 1 : -1;
+    // up: the first entry from q + 2 on of at most `bound`; down: the first from q + 1 back, and
+    // one more
+    auto reach = [&](int bound) {
+      int p = q + 2;
+#pragma unroll
+      for (int lv = kBuildLevels - 1; lv >= 0; --lv) {
+        const int step = d * (1 << lv);
+        if (least(lv, max(p + min(step, 0), 0)) > bound) p += step;
+      }
+      return p;
+    };
+    const int end = reach(min(before, after));
+    if (after == before || end == (d > 0 ? kBuildEnd : 1)) {
+      s_list[atomicAdd(&s_count, 1)] = (uint16_t)q;
+      continue;
+    }
+    // the range's entries are [a, b): its smallest prefix is where it splits
+    const int a = min(q + 2, end), b = max(q + 2, end);
+    const int lv = 31 - __clz(b - a);
+    const int split = reach(min(least(lv, a), least(lv, b - (1 << lv))));
+    out.node(i, n, t0 - 2 + a, t0 - 2 + b, t0 - 2 + split + min(d, 0));
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, part = lane & 7, group = threadIdx.x >> 3;
+  const auto digits = [](int x) { return (31 - __clz(x)) / 3 * 3; };  // 8 << digits exceeds x
+  for (int e0 = group & ~3; e0 < s_count; e0 += kBuildThreads / 8) {  // the same for the warp
+    const int e = e0 + (group & 3), i = t0 + s_list[min(e, s_count - 1)];
+    const int d = lcp(i, i + 1) > lcp(i, i - 1) ? 1 : -1;
+    // how many of the lanes' distances, which rise, still have a prefix above `bound`
+    auto within = [&](long long distance, int bound) {
+      const long long j = i + d * distance;
+      const bool in = j >= 0 && j < n && lcp(i, (int)j) > bound;
+      const uint32_t past = ~__ballot_sync(0xffffffffu, in) >> (lane & 24) & 0xffu;
+      return past ? __ffs(past) - 1 : 8;
+    };
+    // the largest such distance, an octal digit at a time
+    auto reach = [&](int bound, int top) {
+      int l = 0;
+      for (int shift = __reduce_max_sync(0xffffffffu, top); shift >= 0; shift -= 3)
+        l += max(within(l + ((long long)part << shift), bound) - 1, 0) << shift;
+      return l;
+    };
+    const int outside = lcp(i, i - d), c = within(1ll << 3 * part, outside);
+    const int l = reach(outside, c < 8 ? 3 * c - 3 : digits(n)), j = i + d * l;
+    // (the split lies inside the range, whatever unsorted codes say)
+    const int at = min(reach(lcp(i, j), digits(max(l, 1))), max(l - 1, 0));
+    const int split = i + d * at + min(d, 0);
+    if (part == 0 && e < s_count) out.node(i, n, min(i, j), max(i, j), split);
+  }
+}
+
+// A thread per node, searching the codes.
+template <class Lcp>
+__global__ void __launch_bounds__(256) build_few_kernel(Lcp lcp, int n, ar_lbvh::TreeOut out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) parent[n] = -1;  // root: no parent (the reference leaves it unset)
-  if (i >= n - 1) return;
-  ar_lbvh::karras_node(i, n, lcp, is_leaf, left, right, parent, min_r, max_r);
+  if (i == 0) out.parent[n] = -1;
+  if (i < n - 1) ar_lbvh::karras_node(i, n, lcp, out);
+}
+
+// The tiles' barriers and the nodes that leave them cost a small tree more than the searches do:
+// 2,000 points 16.8 us against 15.8, 132,651 points 16.7 against 16.5.
+constexpr int kBuildTilesFrom = 1 << 17;
+template <class Lcp>
+void launch_build(const Lcp& lcp, int n, const ar_lbvh::TreeOut& out, cudaStream_t st) {
+  if (n < kBuildTilesFrom)
+    build_few_kernel<<<arh::grid_for(n - 1, 256), 256, 0, st>>>(lcp, n, out);
+  else
+    build_kernel<<<arh::grid_for(n - 1, kBuildTile), kBuildThreads, 0, st>>>(lcp, n, out);
 }
 
 // ---- leaves (kernelConstructLeafNodesSoA + initializeRadii, BVHSoAKernels.cu:108-138) ------
@@ -439,8 +549,8 @@ ar_status ar_lbvh_build(ar_ctx* ctx, const uint32_t* sorted_codes, int n, uint8_
                                   !min_r || !max_r)))
     return AR_ERR_INVALID_ARG;
   if (n < 2) return AR_OK;
-  build_kernel<<<arh::grid_for(n - 1, 256), 256, 0, arh::stream(stream)>>>(
-      ar_lbvh::Lcp32{sorted_codes, n}, n, is_leaf, left, right, parent, min_r, max_r);
+  launch_build(ar_lbvh::Lcp32{sorted_codes, n}, n,
+               ar_lbvh::TreeOut{is_leaf, left, right, parent, min_r, max_r}, arh::stream(stream));
   return arh::check_launch("ar_lbvh_build");
 }
 
@@ -451,8 +561,8 @@ ar_status ar_lbvh_build64(ar_ctx* ctx, const uint64_t* sorted_codes, int n, uint
                                   !min_r || !max_r)))
     return AR_ERR_INVALID_ARG;
   if (n < 2) return AR_OK;
-  build_kernel<<<arh::grid_for(n - 1, 256), 256, 0, arh::stream(stream)>>>(
-      ar_lbvh::Lcp64{sorted_codes, n}, n, is_leaf, left, right, parent, min_r, max_r);
+  launch_build(ar_lbvh::Lcp64{sorted_codes, n}, n,
+               ar_lbvh::TreeOut{is_leaf, left, right, parent, min_r, max_r}, arh::stream(stream));
   return arh::check_launch("ar_lbvh_build64");
 }
 

@@ -65,12 +65,28 @@ struct Lcp32Scene {
   }
 };
 
-// ---- Karras 2012 internal node i (kernelConstructRadixTreeSoA, BVHSoAKernels.cu:7-99) ----
-// Returns the node's (left, right) child ids.
+// ---- Karras 2012 internal nodes (kernelConstructRadixTreeSoA, BVHSoAKernels.cu:7-99) ----
+struct TreeOut {
+  uint8_t* is_leaf;
+  int32_t *left, *right, *parent, *min_r, *max_r;
+  // Internal node i over the leaves [lo, hi], split after leaf gamma.
+  __device__ __forceinline__ void node(int i, int n, int lo, int hi, int gamma) const {
+    const int node = n + i;
+    is_leaf[node] = 0;
+    const int lc = (lo == gamma) ? gamma : gamma + n;
+    const int rc = (hi == gamma + 1) ? gamma + 1 : gamma + 1 + n;
+    left[node] = lc;
+    right[node] = rc;
+    parent[lc] = node;
+    parent[rc] = node;
+    min_r[node] = lo;
+    max_r[node] = hi;
+  }
+};
+
+// Node i from the sorted codes alone.
 template <class Lcp>
-__device__ __forceinline__ int2 karras_node(int i, int n, const Lcp& lcp, uint8_t* is_leaf,
-                                            int32_t* left, int32_t* right, int32_t* parent,
-                                            int32_t* min_r, int32_t* max_r) {
+__device__ void karras_node(int i, int n, const Lcp& lcp, const TreeOut& out) {
   const int d = (lcp(i, i + 1) - lcp(i, i - 1)) > 0 ? 1 : -1;
   const int sig_min = lcp(i, i - d);
   int lmax = 2;
@@ -90,19 +106,7 @@ __device__ __forceinline__ int2 karras_node(int i, int n, const Lcp& lcp, uint8_
     if (lcp(i, i + (s + t) * d) > sig_node) s += t;
     if (t <= 1) break;
   }
-  const int gamma = i + s * d + min(d, 0);
-  const int node = n + i;
-  const int lo = min(i, j), hi = max(i, j);
-  is_leaf[node] = 0;
-  const int lc = (lo == gamma) ? gamma : gamma + n;
-  const int rc = (hi == gamma + 1) ? gamma + 1 : gamma + 1 + n;
-  left[node] = lc;
-  right[node] = rc;
-  parent[lc] = node;
-  parent[rc] = node;
-  min_r[node] = lo;
-  max_r[node] = hi;
-  return make_int2(lc, rc);
+  out.node(i, n, min(i, j), max(i, j), i + s * d + min(d, 0));
 }
 
 // ---- bottom-up refit (kernelConstructInternalNodesSoA, BVHSoAKernels.cu:148-176) ------------

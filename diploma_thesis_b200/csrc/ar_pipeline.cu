@@ -1290,7 +1290,12 @@ ar_resort::Work resort_work(ar_batch* B, int key_bits) {
   rw.local = B->rs_movers;   // the tiles' movers are dead once grouped by bucket,
   rw.movers = B->rs_movers;  // before the sorted movers are written
   rw.grouped = B->rs_grouped;
-  const int nb_log2 = std::min(ar_resort::kBucketLog2, key_bits);
+  // About 256 particles, a few movers, per bucket: more buckets cost a small scene their scan, fewer
+  // cost a large one their sort (110,592 particles, ten steps: 357 us with 4,096 buckets, 351 with
+  // 2,048, 343 with 512 down to 128, 348 with 64; 2M pile: 1,900 us with 4,096 or 2,048,
+  // 1,912 with 1,024).
+  const int nb_log2 = std::min({ar_resort::kBucketLog2, key_bits,
+                                std::max(5, ceil_log2((uint64_t)B->nt) - 8)});
   rw.nb = 1 << nb_log2;
   rw.bshift = key_bits - nb_log2;
   return rw;

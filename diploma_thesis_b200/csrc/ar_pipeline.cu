@@ -1182,7 +1182,7 @@ ar_status prepare(ar_batch* B, cudaStream_t st) {
               alloc(&B->d_pscene, cn) && alloc(&B->d_bscene, cb) && alloc(&B->pkeys, cn) &&
               alloc(&B->pvals, cn) &&
               alloc(&B->rs_head, ar_resort::region_words(cn)) &&
-              alloc(&B->rs_thead, 2 * ar_resort::tiles_for(cn) + 2) &&
+              alloc(&B->rs_thead, 2 * ar_resort::most_tiles(cn) + 2) &&
               alloc(&B->rs_bstart, (1 << ar_resort::kBucketLog2) + 1) &&
               alloc(&B->rs_movers, cn) && alloc(&B->rs_grouped, cn);
     if (!ok) {
@@ -1263,7 +1263,7 @@ ar_status prepare(ar_batch* B, cudaStream_t st) {
     // so that eight blocks fit on an SM
     static bool carveout_set = false;
     if (!carveout_set) {
-      cudaFuncSetAttribute(ar_resort::place_kernel,
+      cudaFuncSetAttribute(ar_resort::place_kernel<ar_resort::kRowsMany>,
           cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
       cudaGetLastError();
       carveout_set = true;
@@ -1303,20 +1303,27 @@ ar_resort::Work resort_work(ar_batch* B, int key_bits) {
 
 // The four re-sort kernels: B->keys (this step's keys in particle order) from the previous
 // order (pkeys, pvals) into skeys / svals.
-void launch_resort(ar_ctx* ctx, ar_batch* B, const ar_resort::Work& rw, cudaStream_t st) {
+template <int kRows>
+void launch_resort_tiles(ar_ctx* ctx, ar_batch* B, const ar_resort::Work& rw, cudaStream_t st) {
   const int nt = (int)B->nt;
   const unsigned tiles = (unsigned)ar_resort::tiles_for(nt);
   const unsigned wpb = ar_resort::kWarps;  // warps per block: one per tile / bucket
-  arh::launch_pdl(ar_resort::leavers_kernel, dim3(tiles), dim3(ar_resort::kThreads), 0, st,
+  arh::launch_pdl(ar_resort::leavers_kernel<kRows>, dim3(tiles), dim3(ar_resort::kThreads), 0, st,
       (const uint32_t*)B->pkeys, (const uint32_t*)B->pvals, (const uint32_t*)B->keys, nt, rw);
-  arh::launch_pdl(ar_resort::bucket_kernel, dim3((tiles + wpb - 1) / wpb),
+  arh::launch_pdl(ar_resort::bucket_kernel<kRows>, dim3((tiles + wpb - 1) / wpb),
       dim3(ar_resort::kThreads), 0, st, (const uint32_t*)B->pkeys, (const uint32_t*)B->pvals,
       nt, (int)tiles, rw);
   arh::launch_pdl(ar_resort::bucket_sort_kernel, dim3((rw.nb + wpb - 1) / wpb),
       dim3(ar_resort::kThreads), 0, st, rw);
-  arh::launch_pdl(ar_resort::place_kernel, dim3(tiles), dim3(ar_resort::kThreads), 0, st,
+  arh::launch_pdl(ar_resort::place_kernel<kRows>, dim3(tiles), dim3(ar_resort::kThreads), 0, st,
       (const uint32_t*)B->pkeys, (const uint32_t*)B->pvals, nt, rw, B->skeys, B->svals,
       ctx->d_err);
+}
+void launch_resort(ar_ctx* ctx, ar_batch* B, const ar_resort::Work& rw, cudaStream_t st) {
+  if (ar_resort::tile_for(B->nt) == ar_resort::kTileOf<ar_resort::kRowsFew>)
+    launch_resort_tiles<ar_resort::kRowsFew>(ctx, B, rw, st);
+  else
+    launch_resort_tiles<ar_resort::kRowsMany>(ctx, B, rw, st);
 }
 
 // The tree of a BVH step.  32-bit keys leave this step's order for the next step's re-sort.

@@ -7,11 +7,11 @@
 // (old key, index), is almost the new one.  The four kernels below turn it into the new order
 // exactly, whatever the number of particles that moved:
 //
-//   leavers_kernel  over the previous order, one tile of kTile positions per block: a
+//   leavers_kernel  over the previous order, one tile of positions per block: a
 //                   particle whose key changed is a mover; a bit per position marks it, and
 //                   the tile stores its mover count and its movers (new key, index), counted
 //                   per key bucket (key >> bshift).
-//   bucket_kernel   one warp per tile of kTile old positions: the tile's movers into their
+//   bucket_kernel   one warp per tile of old positions: the tile's movers into their
 //                   buckets' ranges, and the tile's header for place_kernel; every block scans
 //                   the bucket counts and the tile counts it needs itself.
 //   bucket_sort_kernel  each bucket sorted by (key, index): one warp per bucket, ranks by
@@ -41,8 +41,14 @@
 namespace ar_resort {
 
 constexpr int kThreads = 256;
-constexpr int kRows = 8;                  // positions per thread and tile
-constexpr int kTile = kThreads * kRows;   // positions of the previous order per tile
+// Positions per thread and tile of the previous order: large tiles cost less per position, small
+// ones spread a small scene over more blocks (step of 110,592 / 216,000 / 373,248 particles 29.7 /
+// 39.3 / 53.5 us with 8 rows, 27.4 / 37.9 / 53.7 with 2; 2M pile 190 / 202 us; 1 and 4 rows
+// measured no better at the first).
+constexpr int kRowsMany = 8, kRowsFew = 2;
+constexpr long kFewBelow = 1l << 18;      // particles
+template <int kRows>
+constexpr int kTileOf = kThreads * kRows;
 constexpr int kWarps = kThreads / 32;
 constexpr int kBucketLog2 = 12;           // at most 2^12 mover buckets
 constexpr int kHeadWords = 4;             // counters at the head of the cleared region
@@ -62,7 +68,7 @@ struct Work {
   uint32_t* tcount;   // movers per tile
   uint4* thead;       // per tile: {w0, w1, movers before the tile, flags}, {previous stayer}
   uint32_t* bstart;   // exclusive prefix of the bucket counts, [nb] = m
-  uint2* local;       // movers of tile t at [t * kTile, t * kTile + tcount[t]), any order
+  uint2* local;       // movers of tile t from its first position on, tcount[t] of them, any order
   uint2* grouped;     // movers grouped by bucket
   uint2* movers;      // movers sorted by (key, index) (may share memory with local)
   int nb;             // buckets (a power of two)
@@ -72,12 +78,19 @@ struct Work {
   __host__ __device__ uint32_t* bfill() const { return head + kHeadWords + kMaxBuckets; }
 };
 
-inline long tiles_for(long n) { return (n + kTile - 1) / kTile; }
+inline int tile_for(long n) { return n < kFewBelow ? kTileOf<kRowsFew> : kTileOf<kRowsMany>; }
+inline long tiles_for(long n) { return (n + tile_for(n) - 1) / tile_for(n); }
+// at most as many tiles for any n up to cap
+inline long most_tiles(long cap) {
+  const long few = cap < kFewBelow ? cap : kFewBelow - 1;
+  const long a = tiles_for(few), b = tiles_for(cap);
+  return a > b ? a : b;
+}
 inline long round4(long x) { return (x + 3) & ~3l; }
 // Layout of the region for a capacity of cap particles; the words the step's first kernel
 // clears.
 inline size_t tcount_offset() { return (size_t)kHeadWords + 2 * (size_t)kMaxBuckets; }
-inline size_t bits_offset(long cap) { return tcount_offset() + round4(tiles_for(cap) + 1); }
+inline size_t bits_offset(long cap) { return tcount_offset() + round4(most_tiles(cap) + 1); }
 inline size_t region_words(long cap) { return bits_offset(cap) + round4(cap / 32 + 1); }
 inline size_t cleared_words() { return tcount_offset(); }
 
@@ -100,6 +113,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 // Stage a tile's old keys, indices (and mover bits) in shared memory: 16-byte copies, positions
 // from n on read as 0.
+template <int kTile>
 __device__ __forceinline__ void stage_tile(const uint32_t* __restrict__ pk,
                                            const uint32_t* __restrict__ pv,
                                            const uint32_t* __restrict__ bits, long base, int n,
@@ -166,16 +180,18 @@ __device__ void block_scan(const uint32_t* a, uint32_t* out, int count) {
 // ---- movers of the previous order -----------------------------------------------------------
 // The tile's old keys and indices are staged in shared memory (asynchronous 16-byte copies), so
 // that few values stay in registers and every tile of the pile runs in one wave.
+template <int kRows>
 __global__ void __launch_bounds__(kThreads, 7) leavers_kernel(
     const uint32_t* __restrict__ pk, const uint32_t* __restrict__ pv,
     const uint32_t* __restrict__ keys, int n, Work w) {
   ar::pdl_wait();
+  constexpr int kTile = kTileOf<kRows>;
   __shared__ __align__(16) uint32_t s_k[kTile];
   __shared__ __align__(16) uint32_t s_v[kTile];
   __shared__ uint32_t s_warp[kWarps];
   const int lane = ar::lane_id(), warp = threadIdx.x >> 5;
   const long base = (long)blockIdx.x * kTile;
-  stage_tile(pk, pv, nullptr, base, n, s_k, s_v, nullptr);
+  stage_tile<kTile>(pk, pv, nullptr, base, n, s_k, s_v, nullptr);
   __syncthreads();
   uint32_t kn[kRows];
 #pragma unroll
@@ -221,10 +237,12 @@ __global__ void __launch_bounds__(kThreads, 7) leavers_kernel(
 // counts before its tiles (and all of them, m); block 0 also stores the bucket starts and m.
 // The loads that do not need the scans (the tile's first 32 movers, its first and last old
 // keys, the last stayer before it) are issued before them.
+template <int kRows>
 __global__ void __launch_bounds__(kThreads) bucket_kernel(const uint32_t* __restrict__ pk,
                                                           const uint32_t* __restrict__ pv,
                                                           int n, int tiles, Work w) {
   ar::pdl_wait();
+  constexpr int kTile = kTileOf<kRows>;
   __shared__ uint32_t s_bstart[(1 << kBucketLog2) + 1];
   __shared__ uint32_t s_red[2][kWarps];
   __shared__ uint32_t s_tc[kWarps];  // movers of the block's tiles
@@ -434,23 +452,26 @@ __global__ void __launch_bounds__(kThreads) bucket_sort_kernel(Work w) {
 // an earlier tile (from the header) and the movers below A are walked down while they lie
 // above it.  Per-position values live in shared memory, not registers, so that every tile of
 // the pile runs in one wave.
+template <int kRows>
 __global__ void __launch_bounds__(kThreads, 7) place_kernel(
     const uint32_t* __restrict__ pk, const uint32_t* __restrict__ pv, int n, Work w,
     uint32_t* __restrict__ out_k, uint32_t* __restrict__ out_v, int* __restrict__ err) {
   ar::pdl_wait();
+  constexpr int kTile = kTileOf<kRows>, kGroups = kRows * kWarps;
+  static_assert(kGroups <= 64, "two groups per lane in the scan");
   __shared__ __align__(16) uint32_t s_k[kTile];     // old keys of the tile
   __shared__ __align__(16) uint32_t s_v[kTile];     // old indices of the tile
   __shared__ __align__(16) uint32_t s_bits[kTile / 32];  // mover bits of the tile
   __shared__ uint32_t s_cnt[kTile];  // movers counted at each stayer, then in-warp prefix
   __shared__ unsigned long long s_win[kWindow];
-  __shared__ uint32_t s_lv[kRows * kWarps];  // movers per (row, warp), then exclusive prefix
-  __shared__ uint32_t s_cs[kRows * kWarps];  // counts per (row, warp), then exclusive prefix
+  __shared__ uint32_t s_lv[kGroups];  // movers per (row, warp), then exclusive prefix
+  __shared__ uint32_t s_cs[kGroups];  // counts per (row, warp), then exclusive prefix
   __shared__ uint32_t s_end;
   const int lane = ar::lane_id(), warp = threadIdx.x >> 5;
   const int tile = blockIdx.x;
   const long base = (long)tile * kTile;
   const int len = (int)(min((long)n, base + kTile) - base);
-  stage_tile(pk, pv, w.bits, base, n, s_k, s_v, s_bits);
+  stage_tile<kTile>(pk, pv, w.bits, base, n, s_k, s_v, s_bits);
   const uint4 h = w.thead[2 * tile];
   const uint32_t m = __ldcg(w.ctr() + 3);
   const uint32_t w0 = min(h.x, m), w1 = max(w0, min(h.y, m));
@@ -500,9 +521,10 @@ __global__ void __launch_bounds__(kThreads, 7) place_kernel(
     }
   }
   __syncthreads();
-  if (threadIdx.x < 32) {  // exclusive prefix sums over the kRows * kWarps = 64 groups
-    const uint32_t c0 = s_lv[2 * lane], c1 = s_lv[2 * lane + 1];
-    const uint32_t d0 = s_cs[2 * lane], d1 = s_cs[2 * lane + 1];
+  if (threadIdx.x < 32) {  // exclusive prefix sums over the (row, warp) groups
+    const bool some = 2 * lane < kGroups;
+    const uint32_t c0 = some ? s_lv[2 * lane] : 0u, c1 = some ? s_lv[2 * lane + 1] : 0u;
+    const uint32_t d0 = some ? s_cs[2 * lane] : 0u, d1 = some ? s_cs[2 * lane + 1] : 0u;
     uint32_t ci = c0 + c1, di = d0 + d1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -514,10 +536,12 @@ __global__ void __launch_bounds__(kThreads, 7) place_kernel(
       }
     }
     const uint32_t cx = ci - c0 - c1, dx = di - d0 - d1;
-    s_lv[2 * lane] = cx;
-    s_lv[2 * lane + 1] = cx + c0;
-    s_cs[2 * lane] = dx;
-    s_cs[2 * lane + 1] = dx + d0;
+    if (some) {
+      s_lv[2 * lane] = cx;
+      s_lv[2 * lane + 1] = cx + c0;
+      s_cs[2 * lane] = dx;
+      s_cs[2 * lane + 1] = dx + d0;
+    }
     if (lane == 31) s_end = w0 + di;
   }
   __syncthreads();

@@ -10,7 +10,7 @@ from diploma_thesis_b200 import api, scenes
 
 pytestmark = pytest.mark.gpu
 
-BLOCK = 2048  # movers a block stages
+BLOCK = 2048  # movers a block stages; the last case has 287,496 particles, in larger tiles
 
 
 def _sorted(gs):
@@ -31,9 +31,9 @@ def _biggest(ka, kb, va, vb, key_bits):
 
 @pytest.mark.parametrize("broadphase", ["grid", "bvh"])
 @pytest.mark.parametrize("side,draw,least", [(2, 0.9, 1), (4, 0.9, 1), (6, 0.9, 1), (9, 0.5, 1),
-                                             (12, 0.1, BLOCK + 1)])
+                                             (12, 0.1, BLOCK + 1), (22, 0.9, 1)])
 def test_bunched_movers(ctx, broadphase, side, draw, least):
-    sc = scenes.small_scene(5, nb_side=side, packed=True, r=1 / 128)
+    sc = scenes.small_scene(5, nb_side=side, packed=True, r=1 / 128 if side < 20 else 1 / 256)
     a = api.GpuScene(ctx, sc, broadphase=broadphase)
     a.step(3)
     (k0, i0, _), _ = _sorted(a)

@@ -1,6 +1,6 @@
 // LBVH device routines shared by the stage entry points (ar_lbvh.cu) and the fused BVH step
 // (ar_pipeline.cu): Karras node construction, fenced bottom-up refit, box tests and the
-// stackless traversal in the reference's visit order.
+// traversal in the reference's visit order.
 //
 // Node numbering is the reference's SoA layout (BVHSource/BVHSoAKernels.cu): leaf i at index
 // i, internal node i at n + i, root at n.  Boxes are the reference's 32-byte AABB

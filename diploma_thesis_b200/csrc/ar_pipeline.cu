@@ -1428,7 +1428,7 @@ ar_status enqueue_step(ar_batch* B, cudaStream_t st, cudaEvent_t* ev = nullptr) 
     AR_LAUNCH_ONE(integrate_kernel, dim3(arh::grid_for(bt, 128)), dim3(128), B->d_table,
         B->d_bscene, bt, B->d_step, ctx->d_err);
     mark(6);
-    B->order_valid = k32;  // the leaves kernel left this step's order in pkeys / pvals
+    B->order_valid = k32;  // the tree kernel left this step's order in pkeys / pvals
     return arh::check_launch("step (BVH)");  // (AR_LAUNCH_ONE is undefined after the grid path)
   }
   // With the last step's order of this particle set at hand, the keys are re-sorted from it
@@ -1627,7 +1627,7 @@ size_t ar_scene_footprint(const ar_scene_desc* d) {
   const size_t shared = 16 /*rel*/ + 16 * 3 /*spos svel pforce*/ + 4 /*svals*/ + 1;
   if (d->broadphase == AR_BROADPHASE_BVH) {
     const size_t per_particle = shared + 8 * 2 /*keys64*/ + 12 /*sort tmp*/ +
-                                2 * (1 + 4 * 5) /*tree*/ + 2 * 32 /*boxes*/ + 4 /*counters*/;
+                                2 * 4 * 3 /*tree*/ + 64 /*wide nodes*/ + 8 + 32 /*open lists*/;
     return n * per_particle + b * per_body + 4096;
   }
   const size_t per_particle = shared + 4 * 2 /*keys*/ + 8 /*sort tmp*/;

@@ -208,8 +208,9 @@ AR_API ar_status ar_lbvh_refit(ar_ctx* ctx, int n, const int32_t* left, const in
  * collideBVHSoARigidBody (Kernels/RB_BVHKernels.cu:100-244) with collideStaticSpheresBVH
  * (:24-98): per sorted leaf, DEM force against every overlapping leaf of another body;
  * p_force4 / p_torque4 / p_positions4 are written at the particle's original index
- * (sorted_idx[leaf]); vel4 is the unsorted particle velocity.  Traversal is stackless
- * (parent links), so no per-thread stack limits the tree depth; `parent` may be NULL (the
+ * (sorted_idx[leaf]); vel4 is the unsorted particle velocity.  Traversal keeps the newest 32
+ * nodes to return to and finds older ones through the parent links, so no per-thread stack
+ * limits the tree depth; `parent` may be NULL (the
  * reference's wrapper signature has none), in which case the links are derived from
  * left/right first.  Contacts are visited in the reference's order. */
 AR_API ar_status ar_collide_bvh_dem(ar_ctx* ctx, const ar_sim_params* params,
@@ -639,8 +640,9 @@ AR_API ar_status ar_scene_destroy_async(ar_scene* scene, ar_stream_t stream);
  * contacts and walls -- the simulateAR branch of updateUniformGridDEM
  * (RigidBodies/UniformGridUpdate.cpp:967-969), which re-sorts the cloud every step; here it
  * is sorted once.  num_points = 0 detaches the cloud.  Synchronises the device (steps in
- * flight may read the old cloud); every batch holding the scene rebuilds its table before
- * its next step.  A clone (ar_scene_clone_async) starts without a cloud.  BVH scenes:
+ * flight may read the old cloud).  A cloud of no more points than the scene's largest so far
+ * is sorted into the buffers the scene has; attaching the first or a larger one, or detaching,
+ * makes every batch holding the scene rebuild its table before its next step.  A clone (ar_scene_clone_async) starts without a cloud.  BVH scenes:
  * AR_ERR_INVALID_ARG. */
 AR_API ar_status ar_scene_set_static_cloud(ar_ctx* ctx, ar_scene* scene, const float* cloud_pos4,
                                            const float* cloud_norm4, int num_points,

@@ -193,8 +193,9 @@ __global__ void __launch_bounds__(kK1Threads) grid_keys_kernel(
 // its own body without loading its occupants (they could only be rejected).  The thread at a
 // cell's first slot writes the whole entry.  The sorted keys and indices are also copied to
 // prev_keys / prev_vals: the order the next step's re-sort starts from.
-// kScatterBatch sorted slots per thread and round, loads issued before use (as in K1).
-constexpr int kScatterBatch = 1;
+// One block per 256 slots: as blocks retire, others start their chain of gathers (a grid of one
+// wave, each thread taking a slot a round, took 2.7 us longer of the 2M
+// pile's 190 us step).
 template <bool kOne>
 __global__ void __launch_bounds__(256) scatter_kernel(
     const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table,
@@ -204,69 +205,35 @@ __global__ void __launch_bounds__(256) scatter_kernel(
     uint32_t* __restrict__ prev_keys, uint32_t* __restrict__ prev_vals,
     const long long* __restrict__ d_step) {
   ar::pdl_wait();
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nt) return;
   const uint32_t epoch = cell_epoch(*d_step) << kEpochShift;
-  const int stride = gridDim.x * blockDim.x;
-  for (int k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < nt; k0 += stride * kScatterBatch) {
-    uint32_t key[kScatterBatch];
-    int g[kScatterBatch], sc[kScatterBatch];
-    bool first[kScatterBatch];
-    float4 r4[kScatterBatch], q[kScatterBatch], c[kScatterBatch], v[kScatterBatch],
-        w[kScatterBatch];
-#pragma unroll
-    for (int u = 0; u < kScatterBatch; ++u) {
-      const int k = k0 + u * stride;
-      if (k < nt) {
-        key[u] = __ldg(skeys + k);
-        g[u] = (int)__ldg(svals + k);
-        first[u] = k == 0 || key[u] != __ldg(skeys + k - 1);
-        prev_keys[k] = key[u];
-        prev_vals[k] = (uint32_t)g[u];
-      }
+  const uint32_t key = __ldg(skeys + k);
+  const int g = (int)__ldg(svals + k);
+  const bool first = k == 0 || key != __ldg(skeys + k - 1);
+  prev_keys[k] = key;
+  prev_vals[k] = (uint32_t)g;
+  const int sc = kOne ? 0 : __ldg(pscene + g);
+  const SceneDev& S = scene_at<kOne>(one, table, sc);
+  const float4 r4 = __ldg(S.rel + (g - S.poff));
+  const int b = __float_as_int(r4.w);
+  const float4 q = __ldg(S.quat + b), c = __ldg(S.pos + b), v = __ldg(S.vel + b),
+               w = __ldg(S.ang + b);
+  if (first) {
+    // occupants of one cell belong to one scene
+    uint32_t tag = body_tag(b);
+    int e = k + 1;
+    for (; e < nt && __ldg(skeys + e) == key; ++e) {
+      const int ge = (int)__ldg(svals + e);
+      if (__float_as_int(__ldg(S.rel + (ge - S.poff)).w) != b) tag = 0;
     }
-#pragma unroll
-    for (int u = 0; u < kScatterBatch; ++u)
-      if (k0 + u * stride < nt) sc[u] = kOne ? 0 : __ldg(pscene + g[u]);
-#pragma unroll
-    for (int u = 0; u < kScatterBatch; ++u) {
-      if (k0 + u * stride < nt) {
-        const SceneDev& S = scene_at<kOne>(one, table, sc[u]);
-        r4[u] = __ldg(S.rel + (g[u] - S.poff));
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kScatterBatch; ++u) {
-      if (k0 + u * stride < nt) {
-        const SceneDev& S = scene_at<kOne>(one, table, sc[u]);
-        const int b = __float_as_int(r4[u].w);
-        q[u] = __ldg(S.quat + b);
-        c[u] = __ldg(S.pos + b);
-        v[u] = __ldg(S.vel + b);
-        w[u] = __ldg(S.ang + b);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kScatterBatch; ++u) {
-      const int k = k0 + u * stride;
-      if (k >= nt) continue;
-      const SceneDev& S = scene_at<kOne>(one, table, sc[u]);
-      const int b = __float_as_int(r4[u].w);
-      if (first[u]) {
-        // occupants of one cell belong to one scene
-        uint32_t tag = body_tag(b);
-        int e = k + 1;
-        for (; e < nt && __ldg(skeys + e) == key[u]; ++e) {
-          const int ge = (int)__ldg(svals + e);
-          if (__float_as_int(__ldg(S.rel + (ge - S.poff)).w) != b) tag = 0;
-        }
-        const uint32_t count = (uint32_t)(e - k) < kCountMask ? (uint32_t)(e - k) : kCountMask;
-        cells[key[u]] = make_uint2((uint32_t)k, count | epoch | (tag << kTagShift));
-      }
-      float3 r, p, vv;
-      ar_pipe::repose(q[u], c[u], v[u], w[u], ar::mk3(r4[u].x, r4[u].y, r4[u].z), &r, &p, &vv);
-      spos[k] = make_float4(p.x, p.y, p.z, __int_as_float(S.boff + b));
-      svel[k] = make_float4(vv.x, vv.y, vv.z, __int_as_float(sc[u]));  // w = scene index
-    }
+    const uint32_t count = (uint32_t)(e - k) < kCountMask ? (uint32_t)(e - k) : kCountMask;
+    cells[key] = make_uint2((uint32_t)k, count | epoch | (tag << kTagShift));
   }
+  float3 r, p, vv;
+  ar_pipe::repose(q, c, v, w, ar::mk3(r4.x, r4.y, r4.z), &r, &p, &vv);
+  spos[k] = make_float4(p.x, p.y, p.z, __int_as_float(S.boff + b));
+  svel[k] = make_float4(vv.x, vv.y, vv.z, __int_as_float(sc));  // w = scene index
 }
 
 // ---- K4: DEM gather + walls ----------------------------------------------------------------
@@ -1458,7 +1425,7 @@ ar_status enqueue_step(ar_batch* B, cudaStream_t st, cudaEvent_t* ev = nullptr) 
     if (s != AR_OK) return s;
   }
   mark(3);
-  AR_LAUNCH_ONE(scatter_kernel, dim3(gp), dim3(256), B->d_table, B->d_pscene, nt, B->skeys,
+  AR_LAUNCH_ONE(scatter_kernel, dim3(arh::grid_for(nt, 256)), dim3(256), B->d_table, B->d_pscene, nt, B->skeys,
       B->svals, B->cells, B->spos, B->svel, B->pkeys, B->pvals, B->d_step);
   mark(4);
   if (nt <= ctx->num_sms * kFewPerSm) {

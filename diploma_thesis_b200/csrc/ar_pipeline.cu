@@ -194,8 +194,7 @@ __global__ void __launch_bounds__(kK1Threads) grid_keys_kernel(
 // cell's first slot writes the whole entry.  The sorted keys and indices are also copied to
 // prev_keys / prev_vals: the order the next step's re-sort starts from.
 // One block per 256 slots: as blocks retire, others start their chain of gathers (a grid of one
-// wave, each thread taking a slot a round, took 2.7 us longer of the 2M
-// pile's 190 us step).
+// wave, each thread taking a slot a round: 2.7 us more of the 2M pile's 190 us step).
 template <bool kOne>
 __global__ void __launch_bounds__(256) scatter_kernel(
     const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table,

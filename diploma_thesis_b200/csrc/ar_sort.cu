@@ -15,8 +15,9 @@
 //     the look-back, so its latency overlaps them;
 //   * items are staged in shared memory in (digit, rank) order and written out with
 //     consecutive threads, so each digit run is a coalesced write.
-// Spin waits are bounded; on timeout the kernel raises kErrTimeout and finishes the pass
-// with whatever prefix it has (the result is then garbage, but nothing hangs).
+// Spin waits are bounded.  A tile whose look-back runs out raises kErrTimeout and counts the digits
+// of all keys before it itself, so the order is right all the same: the kernels behind a sort index
+// with it, and a garbage order would lead them out of their arrays.
 #include <algorithm>
 #include <cuda/atomic>
 #include <mutex>
@@ -226,6 +227,7 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 || kItems < 16 ? 1024 : 51
 
   // look back through the earlier tiles, kLookWindow status words per round trip, until an
   // inclusive prefix is found; then publish this tile's inclusive prefix
+  bool gave_up = false;
   if (d < kDigits) {
     uint32_t excl = 0;
     if (tile != 0) {
@@ -259,13 +261,17 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 || kItems < 16 ? 1024 : 51
         if (!found && used == 0) {
           if (++spins > spin_limit) {
             ar::raise_error(err, ar::kErrTimeout);
+            gave_up = true;
+            excl = 0;
             break;
           }
           if (spins > 64) __nanosleep(64);
         }
       }
-      cuda::atomic_ref<uint32_t, cuda::thread_scope_device> mine(status[(long)tile * kRadix + d]);
-      mine.store(kFlagPrefix | ((excl + tile_count) & kValueMask), cuda::memory_order_relaxed);
+      if (!gave_up) {
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> mine(status[(long)tile * kRadix + d]);
+        mine.store(kFlagPrefix | ((excl + tile_count) & kValueMask), cuda::memory_order_relaxed);
+      }
     }
     sm.gofs[d] = digit_base + excl;
   }
@@ -275,7 +281,20 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 || kItems < 16 ? 1024 : 51
     const long g = wbase + j * 32 + lane;
     if (g < n) sm.vals[rank[j]] = val[j];
   }
-  __syncthreads();
+  if (__syncthreads_or(gave_up)) {  // the block counts the digits before its tile itself
+    uint32_t* before = &sm.warp_hist[0][0];
+    for (int i = tid; i < kDigits; i += kT) before[i] = 0;
+    __syncthreads();
+    for (long i = tid; i < tile_base; i += kT)
+      atomicAdd(before + digit_of(keys_in[i], shift, mask), 1u);
+    __syncthreads();
+    if (gave_up) {
+      cuda::atomic_ref<uint32_t, cuda::thread_scope_device> mine(status[(long)tile * kRadix + d]);
+      mine.store(kFlagPrefix | ((before[d] + tile_count) & kValueMask), cuda::memory_order_relaxed);
+      sm.gofs[d] += before[d];
+    }
+    __syncthreads();
+  }
 
   // coalesced write-out
   long valid = n - tile_base;
@@ -284,7 +303,7 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 || kItems < 16 ? 1024 : 51
     K k = sm.keys[i];
     uint32_t dd = digit_of(k, shift, mask);
     uint32_t dst = sm.gofs[dd] + (uint32_t)i - sm.digit_start[dd];
-    if (dst >= (uint32_t)n) {  // only after a timed-out look-back; never write out of range
+    if (dst >= (uint32_t)n) {  // a histogram that is not the keys'; never write out of range
       ar::raise_error(err, ar::kErrTimeout);
       continue;
     }
@@ -294,9 +313,8 @@ __global__ void __launch_bounds__(kT, (sizeof(K) == 4 || kItems < 16 ? 1024 : 51
 }
 
 // How the digit passes run: ranking by match.any (8-bit digits), the look-back's spin limit,
-// and the failure-detection hook that keeps tile 0 from publishing its status (every later
-// tile's look-back then runs out of spins, reports kErrTimeout and writes nothing out of
-// range).
+// and the failure-detection hook that keeps tile 0 from publishing its status (every look-back that
+// reaches it then runs out of spins, reports kErrTimeout and has its tile count for itself).
 struct PassOpts {
   bool match_rank = false;
   long spin_limit = kSpinLimit;

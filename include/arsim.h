@@ -140,9 +140,10 @@ AR_API ar_status ar_radix_sort_pairs_u64(ar_ctx* ctx, const uint64_t* keys_in,
  *     particles stored body by body), slower when they share many (Morton codes).  The order
  *     is the same.
  *   AR_SORT_TEST_MUTE_FIRST_TILE: failure-detection test hook.  Tile 0 of every digit pass
- *     never publishes its look-back status, and the spin limit drops to 4,096 polls, so every
- *     later tile's look-back gives up: the device error word reports AR_ERR_TIMEOUT (read it
- *     with ar_ctx_status), the outputs are garbage, and nothing is written outside them. */
+ *     never publishes its look-back status, and the spin limit drops to 4,096 polls, so a
+ *     look-back that reaches it gives up: the device error word reports AR_ERR_TIMEOUT (read it
+ *     with ar_ctx_status), and the tile counts the keys before it itself, so that the outputs are
+ *     the sorted pairs all the same. */
 #define AR_SORT_RANK_MATCH 1u
 #define AR_SORT_TEST_MUTE_FIRST_TILE 0x80000000u
 AR_API ar_status ar_radix_sort_pairs_u32_ex(ar_ctx* ctx, const uint32_t* keys_in,

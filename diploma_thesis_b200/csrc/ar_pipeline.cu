@@ -479,15 +479,25 @@ __global__ void __launch_bounds__(256) collide_few_kernel(
 // pLinearImpulse.  Launched only when a scene of the batch has a cloud.
 //
 // A warp owns `per_warp` consecutive sorted particles (a power of two).  First each of its first
-// per_warp lanes finds which of its particle's 27 cells hold points; then the whole warp walks
-// those particles' cells one after another, 32 points at a time: every lane tests a point, the
-// lanes in contact compute their forces together, and the forces are added in the points' order
-// (the shuffles walk the hit mask from its lowest bit), so the sums are the serial ones.  A
-// depth camera puts tens of points in a cell and over a hundred within 2r of a particle, which
-// one thread walked with one dependent round trip after another: bound by that chain (3,200
-// particles on a 640 x 480 cloud: 798 -> 41 us).
+// per_warp lanes finds which of its particle's 27 cells hold points, and how many.  Then either
+// - the whole warp walks those particles' cells one after another, 32 points at a time: every lane
+//   tests a point, the lanes in contact compute their forces together, and the forces are added in
+//   the points' order (the shuffles walk the hit mask from its lowest bit), so the sums are the
+//   serial ones.  A depth camera puts tens of points in a cell and over a hundred within 2r of a
+//   few particles, which one thread walks with one dependent round trip after another: bound by
+//   that chain (3,200 particles on a 640 x 480 cloud: 798 -> 41 us); or
+// - each lane walks its own particle's points, the three cells of an x-row as one run (they are
+//   neighbours in the sorted cloud unless the row wraps), and a contact finds its cell from the
+//   run's inner borders.  With a few points per cell near every particle the warp's walk leaves
+//   most of its lanes idle in each of hundreds of rounds (step of 884,736 particles in a cloud of
+//   2,000,000 points all over the box: 1,608 us with the warp's walk, 391 with the lanes').
+// The warp walks when the longest lane has more than 2/3 as many points to test as the warp takes
+// rounds (its particles' cells, plus a round per 32 points).  With the line at 1 a step with a cloud
+// all over the box gains up to 5 % and one with a sheet loses up to 12 %; with the line at 2/5 clouds
+// of 20 to 30 points per cell lose up to 70 %.
 // per_warp: a scene with few particles spreads them over as many warps as the chip holds, one
 // with many keeps the lanes busy in the first pass, where most particles find no points.
+constexpr float kLaneWalk = 1.5f;  // rounds that a point of the longest lane is worth
 template <bool kOne>
 __global__ void __launch_bounds__(128) cloud_collide_kernel(
     const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table, int nt, int per_warp,
@@ -499,7 +509,7 @@ __global__ void __launch_bounds__(128) cloud_collide_kernel(
   const long k = ((long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane;
   const bool mine = lane < per_warp && k < nt;
   float4 p4 = make_float4(0.f, 0.f, 0.f, 0.f), v4 = p4;
-  uint32_t key = 0, todo = 0;
+  uint32_t key = 0, todo = 0, points = 0;
   if (mine) {
     p4 = __ldg(spos + k);
     v4 = __ldg(svel + k);
@@ -511,8 +521,57 @@ __global__ void __launch_bounds__(128) cloud_collide_kernel(
       for (int r = 0; r < 27; ++r) {
         const uint2 c = __ldg(cc + near_cell(S, key - S.cell_base, r));
         todo |= (c.x < c.y ? 1u : 0u) << r;
+        points += c.y - c.x;
       }
     }
+  }
+  const uint32_t rounds = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(todo) + points / 32);
+  if (rounds == 0) return;
+  if (kLaneWalk * __reduce_max_sync(0xffffffffu, points) <= rounds) {
+    const SceneDev& S = scene_at<kOne>(one, table, kOne ? 0 : __float_as_int(v4.w));
+    const float3 pos = ar::xyz(p4), vel = ar::xyz(v4);
+    const float thr = 2.0f * S.r;
+    const float thr2_up = nextafterf(thr * thr, INFINITY);
+    const uint32_t local = key - S.cell_base, x = local & (S.gx - 1);
+    const bool wraps = x == 0 || x == S.gx - 1;
+    float3 total = ar::mk3(0.f, 0.f, 0.f);
+    const uint32_t some = __reduce_or_sync(0xffffffffu, todo);
+    for (int row = 0; row < 27; row += 3) {
+      if (!((some >> row) & 7u)) continue;
+      for (uint32_t bits = (todo >> row) & 7u; bits;) {
+        const uint32_t take = wraps ? bits & (0u - bits) : bits;
+        bits &= ~take;
+        auto cell = [&](int i) { return __ldg(S.cloud_cells + near_cell(S, local, row + i)); };
+        uint32_t j = cell(__ffs(take) - 1).x;
+        const uint32_t end = cell(31 - __clz(take)).y;
+        const uint32_t second = take & 2u ? cell(1).x : 0xffffffffu;
+        const uint32_t third = take & 4u ? cell(2).x : 0xffffffffu;
+        float3 cf = ar::mk3(0.f, 0.f, 0.f);
+        int cell_now = 0;
+        for (; j < end; ++j) {
+          const float3 rp = ar::sub(ar::xyz(__ldg(S.cloud_pos + j)), pos);
+          const float d2 = ar::dot(rp, rp);
+          if (!(d2 < thr2_up)) continue;
+          const float dist = sqrtf(d2);
+          if (!(dist < thr)) continue;
+          const int c = (j >= second) + 2 * (j >= third);
+          if (c != cell_now) {
+            total = ar::add(total, cf);
+            cf = ar::mk3(0.f, 0.f, 0.f);
+            cell_now = c;
+          }
+          cf = ar::add(cf, ar_dem::scene_force(rp, dist, vel, ar::xyz(__ldg(S.cloud_norm + j)), thr,
+                                               S.k, S.damping, S.shear, S.attraction));
+        }
+        total = ar::add(total, cf);
+      }
+    }
+    if (todo) {
+      float4* f = pforce + __ldg(svals + k);
+      const float4 f0 = *f;
+      *f = make_float4(f0.x + total.x, f0.y + total.y, f0.z + total.z, f0.w);
+    }
+    return;
   }
   for (uint32_t work = __ballot_sync(0xffffffffu, todo != 0); work; work &= work - 1) {
     const int src = __ffs(work) - 1;

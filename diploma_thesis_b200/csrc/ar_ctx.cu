@@ -66,6 +66,10 @@ ar_status check_launch(const char* what) {
   return AR_OK;
 }
 
+namespace {
+size_t arena_size(size_t bytes) { return bytes + bytes / 4 + (1u << 20); }
+}  // namespace
+
 void* scratch(ar_ctx* ctx, size_t bytes) {
   if (bytes <= ctx->scratch_bytes) return ctx->scratch;
   // Growing: the old arena may still be read by queued work, so drain the device first.
@@ -74,13 +78,41 @@ void* scratch(ar_ctx* ctx, size_t bytes) {
   if (ctx->scratch) cudaFree(ctx->scratch);
   ctx->scratch = nullptr;
   ctx->scratch_bytes = 0;
-  size_t grow = bytes + bytes / 4 + (1u << 20);
+  const size_t grow = arena_size(bytes);
   if (dev_malloc(&ctx->scratch, grow) != cudaSuccess) {
     cudaGetLastError();
     set_error("scratch arena: cudaMalloc(%zu) failed", grow);
     return nullptr;
   }
   ctx->scratch_bytes = grow;
+  ctx->reserved = false;
+  return ctx->scratch;
+}
+
+void* scratch(ar_ctx* ctx, size_t need, size_t want, cudaStream_t st) {
+  if (want <= ctx->scratch_bytes) return ctx->scratch;
+  if (need > ctx->scratch_bytes) {
+    void* p = scratch(ctx, want);
+    return p ? p : scratch(ctx, need);
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const bool may_grow = !ctx->reserved && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+                        capture == cudaStreamCaptureStatusNone;
+  if (may_grow) {
+    void* more = nullptr;
+    if (dev_malloc(&more, arena_size(want)) == cudaSuccess) {
+      if (cudaDeviceSynchronize() != cudaSuccess) {  // queued work may still read the old arena
+        cudaFree(more);
+        return nullptr;
+      }
+      cudaFree(ctx->scratch);
+      ctx->scratch = more;
+      ctx->scratch_bytes = arena_size(want);
+      ctx->reserved = false;
+      return more;
+    }
+  }
+  cudaGetLastError();
   return ctx->scratch;
 }
 
@@ -151,7 +183,9 @@ ar_status ar_ctx_destroy(ar_ctx* ctx) {
 
 ar_status ar_ctx_reserve(ar_ctx* ctx, size_t bytes) {
   if (!ctx) return AR_ERR_INVALID_ARG;
-  return arh::scratch(ctx, bytes) ? AR_OK : AR_ERR_OOM;
+  if (!arh::scratch(ctx, bytes)) return AR_ERR_OOM;
+  ctx->reserved = true;
+  return AR_OK;
 }
 
 ar_status ar_ctx_status(ar_ctx* ctx, ar_stream_t stream) {

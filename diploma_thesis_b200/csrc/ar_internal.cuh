@@ -103,12 +103,17 @@ struct ar_ctx {
   int* h_err = nullptr;        // pinned mirror
   void* scratch = nullptr;     // grow-only arena
   size_t scratch_bytes = 0;
+  bool reserved = false;       // the arena's size is what ar_ctx_reserve made it
   int num_sms = 148;
 };
 
 namespace arh {
 // Ensure the context's scratch arena holds at least `bytes`; returns its base or null.
 void* scratch(ar_ctx* ctx, size_t bytes);
+// The arena with `want` bytes if it has them or can be given them, else with `need` or more
+// (ctx->scratch_bytes tells), or null.  An arena that holds `need` is not grown when the caller
+// reserved it or while `st` is being captured, and stays as it is when memory is short.
+void* scratch(ar_ctx* ctx, size_t need, size_t want, cudaStream_t st);
 // Every device and pinned-host allocation of the library goes through these, so that a test
 // can make them fail on the host (ar_test_fail_allocations) and check each AR_ERR_OOM path.
 cudaError_t dev_malloc(void** p, size_t bytes);

@@ -495,14 +495,16 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
 // cubes: 2.47 and 3.57; 3,375 cubes of 8: 3.36 ms with 640).
 constexpr int kSisFew = 256, kSisMany = 640;
 constexpr int kSisManyBodies = 1024;
-constexpr int kMaxSweeps = 32;     // sweeps per schedule (relative velocities kept for each)
+constexpr int kMaxSweeps = 32;     // sweeps per schedule
 constexpr int kLevelChunk = 1024;  // body pairs staged per step of the level walk
 constexpr int kLayoutThreads = 1024;
 constexpr size_t kSisSmemMax = 220 * 1024;   // the sweep block's dynamic shared memory
 constexpr size_t kWalkSmemMax = 200 * 1024;  // the walk's (its static 16 KB stay below 227 KB)
-// The schedule's header in scratch memory: levels, shift, contact count, and whether some contact
-// needs the general update.
-enum { kHdrLevels = 0, kHdrShift = 1, kHdrCount = 2, kHdrGeneral = 3, kHdrWords = 4 };
+// Relative velocities kept at most, 16 bytes each (one per contact and sweep of a schedule).
+constexpr long long kMaxSlots = 1l << 25;
+// The schedule's header in scratch memory: levels, shift, contact count, whether some contact needs
+// the general update, and sweeps per schedule.
+enum { kHdrLevels = 0, kHdrShift = 1, kHdrCount = 2, kHdrGeneral = 3, kHdrSweeps = 4, kHdrWords = 8 };
 
 // Schedule.  Each contact gets a level: 1 + the highest level among earlier contacts on either
 // of its bodies.  Sweep s solves level b at step b + s * shift of one schedule, where shift
@@ -534,8 +536,8 @@ template <bool kShared>
 __global__ void __launch_bounds__(256) sis_levels_kernel(
     const int32_t* __restrict__ body1, const int32_t* __restrict__ body2,
     const int* __restrict__ d_count, int capacity, int num_bodies, int* __restrict__ level,
-    int* __restrict__ last, int* __restrict__ first, int* __restrict__ hdr,
-    int* __restrict__ err) {
+    int* __restrict__ last, int* __restrict__ first, int most_sweeps, long long slots,
+    int* __restrict__ hdr, int* __restrict__ err) {
   extern __shared__ int s_walk[];
   __shared__ int2 s_pair[2][kLevelChunk];
   __shared__ int s_span, s_top;
@@ -615,6 +617,7 @@ __global__ void __launch_bounds__(256) sis_levels_kernel(
     hdr[kHdrShift] = max(4, s_span + 1);
     hdr[kHdrCount] = count;
     hdr[kHdrGeneral] = 0;
+    hdr[kHdrSweeps] = (int)min((long long)most_sweeps, slots / max(count, 1));
   }
 }
 
@@ -702,18 +705,25 @@ __global__ void __launch_bounds__(256) sis_pack_kernel(Contacts C, Bodies B,
   }
 }
 
-// After a schedule of `sweeps` sweeps: the accumulated impulses back to the caller's arrays, and
-// the frictions of the contacts between two bodies, sweep by sweep from the relative velocities
-// that the sweeps kept (the reference accumulates them in its loop; nothing else reads them).
-// The sweep counts start again at zero for the next schedule.
+// The sweeps of the schedule numbered `schedule`, out of `iterations`.
+__device__ __forceinline__ int sweeps_of(int schedule, int iterations, const int* hdr) {
+  const long long left = iterations - (long long)schedule * hdr[kHdrSweeps];
+  return (int)max(0ll, min(left, (long long)hdr[kHdrSweeps]));
+}
+
+// After a schedule: the accumulated impulses back to the caller's arrays, and the frictions of the
+// contacts between two bodies, sweep by sweep from the relative velocities that the sweeps kept
+// (the reference accumulates them in its loop; nothing else reads them).  The sweep counts start
+// again at zero for the next schedule.
 __global__ void __launch_bounds__(256) sis_friction_kernel(Contacts C,
                                                            const Geometry* __restrict__ geo,
                                                            const int* __restrict__ hdr,
                                                            const int* __restrict__ order,
                                                            const float4* __restrict__ vrel,
-                                                           size_t stride, int sweeps,
+                                                           int schedule, int iterations,
                                                            float2* __restrict__ accs) {
-  const int count = hdr[kHdrCount];
+  const int count = hdr[kHdrCount], sweeps = sweeps_of(schedule, iterations, hdr);
+  if (sweeps == 0) return;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
     const int c = order[p];
     const float impulse = accs[2 * (size_t)p].x;
@@ -729,7 +739,7 @@ __global__ void __launch_bounds__(256) sis_friction_kernel(Contacts C,
     const float4 t1 = geo[c].g2, t2 = geo[c].g3;
     float f1 = C.acc_friction[c], f2 = C.acc_friction2[c];
     for (int s = 0; s < sweeps; ++s) {
-      const float3 v = f3(__ldcg(vrel + s * stride + p));
+      const float3 v = f3(__ldcg(vrel + (size_t)s * count + p));
       f1 = clampf(f1 + qdiv(-dot3(v, f3(t1)), t1.w), -bound, bound);
       f2 = clampf(f2 + qdiv(-dot3(v, f3(t2)), t2.w), -bound, bound);
     }
@@ -754,7 +764,7 @@ __device__ __forceinline__ int2 step_range(int step, int levels, int sweeps, int
 // registers of the one it has just solved: its accumulators were last written one step after the
 // last update, shift >= 4 steps before they are needed, so their writer has passed a barrier since.
 template <bool kGeneral, int kThreads>
-__device__ __forceinline__ void run_schedule(int levels, int shift, int capacity, int sweeps,
+__device__ __forceinline__ void run_schedule(int levels, int shift, int stride, int sweeps,
                                              float upper_bound, const int2* runs,
                                              const float4* rec, float2* accs, float4* vel,
                                              float4* ang, float4* vrel, int2* s_range) {
@@ -768,11 +778,11 @@ __device__ __forceinline__ void run_schedule(int levels, int shift, int capacity
   };
   auto solve = [&](Half& it, int2 r, int2 ahead) {
     if (__any_sync(0xffffffffu, it.h >= 0 || rest.h >= 0)) {
-      solve_half<kGeneral>(it, accs, vel, ang, vrel, capacity, upper_bound, rest);
+      solve_half<kGeneral>(it, accs, vel, ang, vrel, stride, upper_bound, rest);
       for (int h0 = 2 * r.x + kThreads; h0 < 2 * r.y; h0 += kThreads) {
         // contacts beyond one per lane pair
         load_half(rec, accs, h0 + lane < 2 * r.y ? h0 + lane : -1, it);
-        solve_half<kGeneral>(it, accs, vel, ang, vrel, capacity, upper_bound, rest);
+        solve_half<kGeneral>(it, accs, vel, ang, vrel, stride, upper_bound, rest);
       }
     }
     fetch(ahead, it);
@@ -795,7 +805,7 @@ __device__ __forceinline__ void run_schedule(int levels, int shift, int capacity
       solve(b, s_range[i + 1], s_range[i + 3]);
     }
   }
-  store_rest(rest, accs, vrel, capacity);
+  store_rest(rest, accs, vrel, stride);
 }
 
 // The sweeps, in one block.  kShared: the bodies' velocities and angular velocities live in shared
@@ -810,12 +820,14 @@ __device__ __forceinline__ void run_schedule(int levels, int shift, int capacity
 // instructions: 9.7 ms); three register buffers (spills: 28 ms).
 template <bool kShared, int kThreads>
 __global__ void __launch_bounds__(kThreads) sis_sweep_kernel(
-    Bodies B, const int* __restrict__ hdr, int capacity, int num_bodies, int sweeps,
+    Bodies B, const int* __restrict__ hdr, int num_bodies, int schedule, int iterations,
     float upper_bound, const int2* __restrict__ run, const float4* __restrict__ rec,
     float2* __restrict__ accs, float4* __restrict__ vrel) {
   extern __shared__ float4 s_bodies[];  // (kShared) vel[num_bodies], ang[num_bodies]
   __shared__ int2 s_range[kThreads];
-  const int levels = hdr[kHdrLevels], shift = hdr[kHdrShift];
+  const int levels = hdr[kHdrLevels], shift = hdr[kHdrShift], count = hdr[kHdrCount];
+  const int sweeps = sweeps_of(schedule, iterations, hdr);
+  if (sweeps == 0) return;
   float4 *vel = B.vel, *ang = B.ang;
   if (kShared) {
     vel = s_bodies;
@@ -828,10 +840,10 @@ __global__ void __launch_bounds__(kThreads) sis_sweep_kernel(
   __syncthreads();
   if (levels > 0) {
     if (hdr[kHdrGeneral])
-      run_schedule<true, kThreads>(levels, shift, capacity, sweeps, upper_bound, run, rec, accs,
+      run_schedule<true, kThreads>(levels, shift, count, sweeps, upper_bound, run, rec, accs,
                                    vel, ang, vrel, s_range);
     else
-      run_schedule<false, kThreads>(levels, shift, capacity, sweeps, upper_bound, run, rec, accs,
+      run_schedule<false, kThreads>(levels, shift, count, sweeps, upper_bound, run, rec, accs,
                                     vel, ang, vrel, s_range);
   }
   if (kShared) {
@@ -920,34 +932,42 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
     arh::set_error("iterations x (capacity + 1) must stay below 2^31");
     return AR_ERR_INVALID_ARG;
   }
-  // scratch: geometry[capacity] (64-byte aligned), the halves' records (word-major), the relative
-  // velocities of a schedule's sweeps, the accumulators, level runs run[capacity + 1], the
-  // schedule header, then level[capacity], order[capacity], last[num_bodies], first[num_bodies]
-  const int batch = std::min(iterations, kMaxSweeps);
+  // scratch: geometry[capacity] (64-byte aligned), the halves' records (word-major), the
+  // accumulators, level runs run[capacity + 1], the schedule header, level[capacity],
+  // order[capacity], last[num_bodies], first[num_bodies], then the relative velocities of a
+  // schedule's sweeps.  These get room for all sweeps of `capacity` contacts, up to kMaxSlots, and
+  // at least for one; the contacts that there are take what sweeps fit (kHdrSweeps), since the
+  // results do not depend on where the sweeps are cut into schedules.
   const size_t cap = (size_t)capacity;
   const size_t geo_bytes = sizeof(Geometry) * cap;
   const size_t rec_bytes = sizeof(float4) * ((2 * cap + 31) / 32 * 32) * kHalfWords;
-  const size_t vrel_bytes = sizeof(float4) * cap * batch;
   const size_t acc_bytes = sizeof(float2) * 2 * cap;
   const size_t run_bytes = sizeof(int2) * (cap + 1);
   const size_t words = kHdrWords + 2 * cap + 2 * (size_t)num_bodies;
-  char* base = (char*)arh::scratch(ctx, geo_bytes + rec_bytes + vrel_bytes + acc_bytes +
-                                            run_bytes + sizeof(int) * words);
+  const size_t fixed_bytes =
+      (geo_bytes + rec_bytes + acc_bytes + run_bytes + sizeof(int) * words + 15) & ~(size_t)15;
+  const int most_sweeps = std::min(iterations, kMaxSweeps);
+  const long long want_slots =
+      std::max((long long)capacity, std::min((long long)capacity * most_sweeps, kMaxSlots));
+  cudaStream_t st = arh::stream(stream);
+  char* base = (char*)arh::scratch(ctx, fixed_bytes + sizeof(float4) * cap,
+                                   fixed_bytes + sizeof(float4) * (size_t)want_slots, st);
   if (!base) return AR_ERR_OOM;
+  const long long slots =
+      std::min(want_slots, (long long)((ctx->scratch_bytes - fixed_bytes) / sizeof(float4)));
   Geometry* geo = (Geometry*)base;
   float4* rec = (float4*)(base + geo_bytes);
-  float4* vrel = (float4*)((char*)rec + rec_bytes);
-  float2* accs = (float2*)(vrel + cap * batch);
+  float2* accs = (float2*)((char*)rec + rec_bytes);
   int2* run = (int2*)(accs + 2 * cap);
   int* hdr = (int*)(run + cap + 1);
   int* level = hdr + kHdrWords;
   int* order = level + capacity;
   int* last = order + capacity;
   int* first = last + num_bodies;
+  float4* vrel = (float4*)(base + fixed_bytes);
   Contacts C{(const float4*)normal4, (const float4*)point4, body1, body2, bias, acc_impulse,
              acc_friction, acc_friction2};
   Bodies B{(const float4*)cms4, (float4*)vel4, (float4*)ang4, cur_inv_inertia9, mass};
-  cudaStream_t st = arh::stream(stream);
   const unsigned gg = std::min(arh::grid_for(capacity, 256), (unsigned)ctx->num_sms * 8);
   sis_geometry_kernel<<<gg, 256, 0, st>>>(C, B, d_count, capacity, params->ar_friction,
                                           params->rb_friction, fabsf(params->gravity[1]), geo);
@@ -958,11 +978,12 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
     cudaFuncSetAttribute(sis_levels_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)walk_smem);
     sis_levels_kernel<true><<<1, 256, walk_smem, st>>>(body1, body2, d_count, capacity,
-                                                      num_bodies, level, last, first, hdr,
-                                                      ctx->d_err);
+                                                      num_bodies, level, last, first,
+                                                      most_sweeps, slots, hdr, ctx->d_err);
   } else {
     sis_levels_kernel<false><<<1, 256, 0, st>>>(body1, body2, d_count, capacity, num_bodies,
-                                               level, last, first, hdr, ctx->d_err);
+                                               level, last, first, most_sweeps, slots, hdr,
+                                               ctx->d_err);
   }
   sis_sizes_kernel<<<gg, 256, 0, st>>>(level, hdr, run);
   sis_layout_kernel<<<1, kLayoutThreads, 0, st>>>(hdr, run, order);
@@ -976,11 +997,12 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
   auto* sweep = !shared ? sis_sweep_kernel<false, kSisMany>
                         : (many ? sis_sweep_kernel<true, kSisMany> : sis_sweep_kernel<true, kSisFew>);
   cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  for (int done = 0; done < iterations; done += batch) {
-    const int sweeps = std::min(batch, iterations - done);
+  // as many schedules as `capacity` contacts take; with fewer the last ones find no sweeps left
+  const int fewest = (int)std::min((long long)most_sweeps, slots / capacity);
+  for (int i = 0; i * (long long)fewest < iterations; ++i) {
     sweep<<<1, !shared || many ? kSisMany : kSisFew, smem, st>>>(
-        B, hdr, capacity, num_bodies, sweeps, 100.f, run, rec, accs, vrel);
-    sis_friction_kernel<<<gg, 256, 0, st>>>(C, geo, hdr, order, vrel, cap, sweeps, accs);
+        B, hdr, num_bodies, i, iterations, 100.f, run, rec, accs, vrel);
+    sis_friction_kernel<<<gg, 256, 0, st>>>(C, geo, hdr, order, vrel, i, iterations, accs);
   }
   return arh::check_launch("ar_sequential_impulse");
 }

@@ -82,7 +82,8 @@ AR_API ar_status ar_ctx_destroy(ar_ctx* ctx);
  * call: AR_ERR_TIMEOUT, AR_ERR_NAN, AR_ERR_OVERFLOW or AR_OK.  Replaces checkCudaErrors'
  * exit() (Libs/common/inc/helper_cuda.h:967-981). */
 AR_API ar_status ar_ctx_status(ar_ctx* ctx, ar_stream_t stream);
-/* Pre-size the scratch arena (so later calls inside a CUDA graph capture never grow it). */
+/* Pre-size the scratch arena (so later calls inside a CUDA graph capture never grow it).  A call
+ * that can do with what the arena holds does not grow a reserved one. */
 AR_API ar_status ar_ctx_reserve(ar_ctx* ctx, size_t bytes);
 AR_API const char* ar_last_error(void);
 AR_API const char* ar_version(void);
@@ -551,7 +552,9 @@ AR_API ar_status ar_gather_contacts(ar_ctx* ctx, const ar_sim_params* params, in
  * body are solved together, one dependency level at a time, in one thread block, and later
  * sweeps start before earlier ones end wherever no body is shared (each body still sees the
  * loop's order of updates).  iterations x (capacity + 1) must stay below 2^31
- * (AR_ERR_INVALID_ARG otherwise). */
+ * (AR_ERR_INVALID_ARG otherwise).  Scratch: 272 bytes per contact slot, 8 per body and 4 KB do; with
+ * 16 more bytes per contact and sweep (the arena takes up to 512 MB for them when it has to grow
+ * anyway, and if it can) all sweeps go into one schedule, which is faster. */
 AR_API ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params,
                                        const int32_t* d_count, int capacity,
                                        const float* normal4, const float* point4,

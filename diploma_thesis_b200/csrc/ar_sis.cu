@@ -495,7 +495,6 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
 // cubes: 2.47 and 3.57; 3,375 cubes of 8: 3.36 ms with 640).
 constexpr int kSisFew = 256, kSisMany = 640;
 constexpr int kSisManyBodies = 1024;
-constexpr int kMaxSweeps = 32;     // sweeps per schedule
 constexpr int kLevelChunk = 1024;  // body pairs staged per step of the level walk
 constexpr int kLayoutThreads = 1024;
 constexpr size_t kSisSmemMax = 220 * 1024;   // the sweep block's dynamic shared memory
@@ -536,7 +535,7 @@ template <bool kShared>
 __global__ void __launch_bounds__(256) sis_levels_kernel(
     const int32_t* __restrict__ body1, const int32_t* __restrict__ body2,
     const int* __restrict__ d_count, int capacity, int num_bodies, int* __restrict__ level,
-    int* __restrict__ last, int* __restrict__ first, int most_sweeps, long long slots,
+    int* __restrict__ last, int* __restrict__ first, int iterations, long long slots,
     int* __restrict__ hdr, int* __restrict__ err) {
   extern __shared__ int s_walk[];
   __shared__ int2 s_pair[2][kLevelChunk];
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(256) sis_levels_kernel(
     hdr[kHdrShift] = max(4, s_span + 1);
     hdr[kHdrCount] = count;
     hdr[kHdrGeneral] = 0;
-    hdr[kHdrSweeps] = (int)min((long long)most_sweeps, slots / max(count, 1));
+    hdr[kHdrSweeps] = (int)min((long long)iterations, slots / max(count, 1));
   }
 }
 
@@ -946,9 +945,8 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
   const size_t words = kHdrWords + 2 * cap + 2 * (size_t)num_bodies;
   const size_t fixed_bytes =
       (geo_bytes + rec_bytes + acc_bytes + run_bytes + sizeof(int) * words + 15) & ~(size_t)15;
-  const int most_sweeps = std::min(iterations, kMaxSweeps);
   const long long want_slots =
-      std::max((long long)capacity, std::min((long long)capacity * most_sweeps, kMaxSlots));
+      std::max((long long)capacity, std::min((long long)capacity * iterations, kMaxSlots));
   cudaStream_t st = arh::stream(stream);
   char* base = (char*)arh::scratch(ctx, fixed_bytes + sizeof(float4) * cap,
                                    fixed_bytes + sizeof(float4) * (size_t)want_slots, st);
@@ -979,10 +977,10 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
                          (int)walk_smem);
     sis_levels_kernel<true><<<1, 256, walk_smem, st>>>(body1, body2, d_count, capacity,
                                                       num_bodies, level, last, first,
-                                                      most_sweeps, slots, hdr, ctx->d_err);
+                                                      iterations, slots, hdr, ctx->d_err);
   } else {
     sis_levels_kernel<false><<<1, 256, 0, st>>>(body1, body2, d_count, capacity, num_bodies,
-                                               level, last, first, most_sweeps, slots, hdr,
+                                               level, last, first, iterations, slots, hdr,
                                                ctx->d_err);
   }
   sis_sizes_kernel<<<gg, 256, 0, st>>>(level, hdr, run);
@@ -998,7 +996,7 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
                         : (many ? sis_sweep_kernel<true, kSisMany> : sis_sweep_kernel<true, kSisFew>);
   cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // as many schedules as `capacity` contacts take; with fewer the last ones find no sweeps left
-  const int fewest = (int)std::min((long long)most_sweeps, slots / capacity);
+  const int fewest = (int)std::min((long long)iterations, slots / capacity);
   for (int i = 0; i * (long long)fewest < iterations; ++i) {
     sweep<<<1, !shared || many ? kSisMany : kSisFew, smem, st>>>(
         B, hdr, num_bodies, i, iterations, 100.f, run, rec, accs, vrel);

@@ -395,7 +395,8 @@ __device__ __forceinline__ void load_half(const float4* rec, const float2* accs,
 // lanes that hold its halves (every lane of the warp calls it).  Each lane takes its body's share
 // of the relative velocity, both compute the impulse, and each updates its body.  Friction between
 // two bodies is accumulated but never applied (as in the reference), so only the relative velocity
-// it needs is kept, in `vrel`, for sis_friction_kernel.  kGeneral: some contact of the list has one
+// it needs is kept, in `vrel`, for sis_friction_kernel.  Lanes without a contact compute along on
+// what their registers hold, so they must not decide on a warp's plain division.  kGeneral: some contact of the list has one
 // body, or one body twice, or a divisor outside div_by's range.
 // What an update leaves to be stored: no other update waits for it, so it is done in the next
 // step, between that step's dependent operations.
@@ -445,7 +446,7 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
     change = qdiv(x, mc);
   } else {
     change = div_by(x, mc, side ? it.acc.x : met);
-    if (!div_dividend(x)) change = x / mc;
+    if (have && !div_dividend(x)) change = x / mc;
   }
   const float total = clampf(acc + change, 0.f, upper_bound);
   float3 imp = mul3(total - acc, n);
@@ -476,7 +477,7 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
   } else {
     const float rm = it.w[4].z;
     dv = ar::mk3(div_by(imp.x, m, rm), div_by(imp.y, m, rm), div_by(imp.z, m, rm));
-    if (!(div_dividend(imp.x) && div_dividend(imp.y) && div_dividend(imp.z)))
+    if (have && !(div_dividend(imp.x) && div_dividend(imp.y) && div_dividend(imp.z)))
       dv = ar::mk3(imp.x / m, imp.y / m, imp.z / m);
   }
   const float I[9] = {it.w[2].x, it.w[2].y, it.w[2].z, it.w[2].w, it.w[3].x,

@@ -317,15 +317,20 @@ __device__ __forceinline__ bool div_divisor(float d) {  // 2^-40 <= |d| < 2^40
 // The second half's inverse inertia, mass and 1 / mass are negated: its body takes the opposite
 // impulse, and negated factors give exactly the negated products, sums and quotients.
 // A contact with one body has no second half; its place holds what the first one's friction needs:
-//   t1, k1 | t2, k2 | - | - | friction bound, -, -, flags
+//   t1, k1 | t2, k2 | 1 / mc, 1 / k1, 1 / k2, - | - | friction bound, 0, 0, kNoBody
 // Beside them two floats per half that change: the impulse and the number of sweeps done (first
 // half); 1 / mc, or a one-body contact's two frictions (second half).
+// kOdd marks the contacts that the plain form of solve_half does not cover: those with one body,
+// with one body twice, or with a divisor outside div_by's range, whose reciprocal is a NaN here.
 constexpr int kHalfWords = 5;
-constexpr uint32_t kOneBody = 1u << 31, kSelfPair = 1u << 30, kBodyMask = kSelfPair - 1;  // flags
+constexpr uint32_t kOdd = 1u << 31, kNoBody = 0xffffffffu;
+__device__ __forceinline__ float reciprocal(float d) {
+  return div_divisor(d) ? 1.0f / d : __int_as_float(0x7fc00000);
+}
 __device__ __forceinline__ size_t half_at(int h) {
   return (size_t)(h >> 5) * (32 * kHalfWords) + (h & 31);
 }
-// Returns whether the contact needs the general form of solve_half.
+// Returns whether the contact is odd.
 __device__ __forceinline__ bool pack_contact(const Contacts& C, const Bodies& B,
                                              const Geometry* __restrict__ geo, int c, int p,
                                              float4* __restrict__ rec,
@@ -333,34 +338,35 @@ __device__ __forceinline__ bool pack_contact(const Contacts& C, const Bodies& B,
   const int i1 = C.body1[c], i2 = C.body2[c];
   const float4 n = C.normal[c];
   const Geometry g = geo[c];
-  const uint32_t flags = i2 < 0 ? kOneBody : (i2 == i1 ? kSelfPair : 0u);
-  bool general = flags != 0u || !div_divisor(g.g0.w);
-  auto half = [&](int side, float4 arm, int body) {
-    const float sign = side ? -1.f : 1.f, m = sign * B.mass[body];
+  const float mc = g.g0.w, m1 = B.mass[i1], m2 = i2 >= 0 ? B.mass[i2] : m1;
+  const bool odd = i2 < 0 || i2 == i1 || !div_divisor(mc) || !div_divisor(m1) || !div_divisor(m2);
+  auto half = [&](int side, float4 arm, int body, float mass) {
+    const float sign = side ? -1.f : 1.f, m = sign * mass;
     float I[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) I[k] = sign * B.inv_inertia[9 * body + k];
+    for (int k = 0; k < 9; ++k) I[k] = sign * B.inv_inertia[9 * (size_t)body + k];
     float4* out = rec + half_at(2 * p + side);
     out[0] = make_float4(n.x, n.y, n.z, C.bias[c]);
-    out[32] = make_float4(arm.x, arm.y, arm.z, g.g0.w);
+    out[32] = make_float4(arm.x, arm.y, arm.z, mc);
     out[64] = make_float4(I[0], I[1], I[2], I[3]);
     out[96] = make_float4(I[4], I[5], I[6], I[7]);
-    out[128] = make_float4(I[8], m, 1.0f / m, __uint_as_float((uint32_t)body | flags));
-    general |= !div_divisor(m);
+    out[128] = make_float4(I[8], m, reciprocal(m),
+                           __uint_as_float((uint32_t)body | (odd ? kOdd : 0u)));
   };
-  half(0, g.g0, i1);
+  half(0, g.g0, i1, m1);
   if (i2 >= 0) {
-    half(1, g.g1, i2);
+    half(1, g.g1, i2, m2);
   } else {
     float4* out = rec + half_at(2 * p + 1);
     out[0] = g.g2;
     out[32] = g.g3;
-    out[128] = make_float4(g.g1.w, 0.f, 0.f, __uint_as_float(flags));
+    out[64] = make_float4(reciprocal(mc), reciprocal(g.g2.w), reciprocal(g.g3.w), 0.f);
+    out[128] = make_float4(g.g1.w, 0.f, 0.f, __uint_as_float(kNoBody));
   }
   accs[2 * (size_t)p] = make_float2(C.acc_impulse[c], __int_as_float(0));
-  accs[2 * (size_t)p + 1] = i2 >= 0 ? make_float2(1.0f / g.g0.w, 0.f)
+  accs[2 * (size_t)p + 1] = i2 >= 0 ? make_float2(reciprocal(mc), 0.f)
                                     : make_float2(C.acc_friction[c], C.acc_friction2[c]);
-  return general;
+  return odd;
 }
 
 // Half of a contact, held in registers (h: its place, -1: none).
@@ -398,8 +404,8 @@ __device__ __forceinline__ void load_half(const float4* rec, const float2* accs,
 // of the relative velocity, both compute the impulse, and each updates its body.  Friction between
 // two bodies is accumulated but never applied (as in the reference), so only the relative velocity
 // it needs is kept, in `vrel`, for sis_friction_kernel.  Lanes without a contact compute along on
-// what their registers hold, so they must not decide on a warp's plain division.  kGeneral: some contact of the list has one
-// body, or one body twice, or a divisor outside div_by's range.
+// what their registers hold, so they must not decide on a warp's plain division.  kGeneral: some
+// contact of the list is odd (else the compiler leaves the tests for it out).
 // What an update leaves to be stored: no other update waits for it, so it is done in the next
 // step, between that step's dependent operations.
 struct Rest {
@@ -427,65 +433,69 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
   const bool side = threadIdx.x & 1;
   const bool have = it.h >= 0;
   const uint32_t tag = have ? __float_as_uint(it.w[4].w) : 0u;
-  const bool one = kGeneral && (tag & kOneBody);
-  const bool mine = have && !(one && side);  // this lane holds a body
-  const int body = mine ? (int)(tag & kBodyMask) : 0;
+  const bool mine = have && tag != kNoBody;  // this lane holds a body
+  const int body = mine ? (int)(tag & ~kOdd) : 0;
   const float3 n = f3(it.w[0]), arm = f3(it.w[1]);
   const float mc = it.w[1].w, m = it.w[4].y;
   const float3 v = f3(vel[body]), w = f3(ang[body]);
+  // of a general list, the warps with an odd contact (the whole warp takes a branch on `some`)
+  const bool odd = kGeneral && (tag & kOdd);
+  const bool some = kGeneral && __any_sync(kAll, odd);
+  const uint32_t other = some ? __shfl_xor_sync(kAll, tag, 1) : tag;
+  const bool one = odd && (side ? tag : other) == kNoBody;
   store_rest(rest, accs, vrel, stride);  // the previous update's
   // the first lane's impulse against the second one's 1 / mc
   const float met = __shfl_xor_sync(kAll, it.acc.x, 1);
   const float acc = side ? met : it.acc.x;
+  float rmc = side ? it.acc.x : met;
+  if (some) {
+    const float r = __shfl_xor_sync(kAll, it.w[2].x, 1);
+    if (one) rmc = r;
+  }
   const float3 c = cross3(w, arm);
   const float3 at = add3(v, c);  // the body's velocity at the contact
   const float s = dot3(at, n);
   const float d = s - __shfl_xor_sync(kAll, s, 1);
   const float v_rel = one ? s : (side ? -d : d);
   const float x = -(v_rel + it.w[0].w);
-  float change;
-  if (kGeneral) {
-    change = qdiv(x, mc);
-  } else {
-    change = div_by(x, mc, side ? it.acc.x : met);
-    if (have && !div_dividend(x)) change = x / mc;
-  }
+  float change = div_by(x, mc, rmc);
+  if (mine && !(div_dividend(x) && (!kGeneral || rmc == rmc))) change = x / mc;
   const float total = clampf(acc + change, 0.f, upper_bound);
   float3 imp = mul3(total - acc, n);
-  if (kGeneral && __any_sync(kAll, one)) {
+  if (some) {
     // one body: the second lane computes the frictions, which are applied
     auto pair = [&](float3 a) {  // the other half's
       return ar::mk3(__shfl_xor_sync(kAll, a.x, 1), __shfl_xor_sync(kAll, a.y, 1),
                      __shfl_xor_sync(kAll, a.z, 1));
     };
     const float3 vel1 = pair(at);
-    float cf1 = 0.f, cf2 = 0.f;
-    if (one && side) {
-      const float bound = it.w[4].x;
-      cf1 = qdiv(-dot3(vel1, f3(it.w[0])), it.w[0].w);
-      const float f1 = clampf(it.acc.x + cf1, -bound, bound);
-      cf1 = f1 - it.acc.x;
-      cf2 = qdiv(-dot3(vel1, f3(it.w[1])), it.w[1].w);
-      const float f2 = clampf(it.acc.y + cf2, -bound, bound);
-      cf2 = f2 - it.acc.y;
-      accs[it.h] = make_float2(f1, f2);
+    const bool friction = one && side;
+    const float x1 = -dot3(vel1, n), x2 = -dot3(vel1, arm);  // along t1 and t2
+    float cf1 = div_by(x1, it.w[0].w, it.w[2].y), cf2 = div_by(x2, mc, it.w[2].z);
+    if (friction && !(div_dividend(x1) && div_dividend(x2) && it.w[2].y == it.w[2].y &&
+                      it.w[2].z == it.w[2].z)) {
+      cf1 = x1 / it.w[0].w;
+      cf2 = x2 / mc;
     }
-    const float3 fx = pair(mul3(cf1, f3(it.w[0]))), fy = pair(mul3(cf2, f3(it.w[1])));
+    const float bound = it.w[4].x;
+    const float f1 = clampf(it.acc.x + cf1, -bound, bound);
+    cf1 = f1 - it.acc.x;
+    const float f2 = clampf(it.acc.y + cf2, -bound, bound);
+    cf2 = f2 - it.acc.y;
+    if (friction) accs[it.h] = make_float2(f1, f2);
+    const float3 fx = pair(mul3(cf1, n)), fy = pair(mul3(cf2, arm));
     if (one) imp = add3(add3(imp, fx), fy);
   }
-  float3 dv;
-  if (kGeneral) {
-    dv = qdiv3(imp, m);
-  } else {
-    const float rm = it.w[4].z;
-    dv = ar::mk3(div_by(imp.x, m, rm), div_by(imp.y, m, rm), div_by(imp.z, m, rm));
-    if (have && !(div_dividend(imp.x) && div_dividend(imp.y) && div_dividend(imp.z)))
-      dv = ar::mk3(imp.x / m, imp.y / m, imp.z / m);
-  }
+  const float rm = it.w[4].z;
+  float3 dv = ar::mk3(div_by(imp.x, m, rm), div_by(imp.y, m, rm), div_by(imp.z, m, rm));
+  if (mine && !(div_dividend(imp.x) && div_dividend(imp.y) && div_dividend(imp.z) &&
+                (!kGeneral || rm == rm)))
+    dv = ar::mk3(imp.x / m, imp.y / m, imp.z / m);
   const float I[9] = {it.w[2].x, it.w[2].y, it.w[2].z, it.w[2].w, it.w[3].x,
                       it.w[3].y, it.w[3].z, it.w[3].w, it.w[4].x};
   const float3 nv = add3(v, dv), nw = add3(w, mv(I, cross3(arm, imp)));
-  if (mine && (!kGeneral || side || !(tag & kSelfPair))) {  // a self pair: the second half stands
+  // of a contact of one body with itself the second half's update stands
+  if (mine && (side || !odd || tag != other)) {
     vel[body] = make_float4(nv.x, nv.y, nv.z, 0.f);
     ang[body] = make_float4(nw.x, nw.y, nw.z, 0.f);
   }

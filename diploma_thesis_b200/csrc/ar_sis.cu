@@ -502,12 +502,9 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
   rest = Rest{it.h, __float_as_int(it.acc.y), total, v, c};
 }
 
-// Threads of the sweep block, two lanes per contact, and the bodies from which it has the larger
-// number: a step holds more contacts the more bodies there are (512 cubes: 54 at most, 4,096: 282),
-// and idle warps cost every step a little (512 cubes: 3.78 ms with 256 threads, 4.04 with 640; 27
-// cubes: 2.47 and 3.57; 3,375 cubes of 8: 3.36 ms with 640).
-constexpr int kSisFew = 256, kSisMany = 640;
-constexpr int kSisManyBodies = 1024;
+// Threads of the sweep block, two lanes per contact: a step's first 320 contacts are loaded ahead.
+// The block keeps as many warps as its widest step fills; idle ones would cost every step a little.
+constexpr int kSisThreads = 640;
 constexpr int kLevelChunk = 1024;  // body pairs staged per step of the level walk
 constexpr int kLayoutThreads = 1024;
 constexpr size_t kSisSmemMax = 220 * 1024;   // the sweep block's dynamic shared memory
@@ -771,17 +768,23 @@ __device__ __forceinline__ int2 step_range(int step, int levels, int sweeps, int
   return lo <= hi && hi >= 1 ? make_int2(runs[lo].y, runs[hi].x) : make_int2(0, 0);
 }
 
+// Barrier of the block's first `lanes` threads.
+__device__ __forceinline__ void lanes_barrier(int lanes) {
+  asm volatile("bar.sync 1, %0;" ::"r"(lanes) : "memory");
+}
+
 // The steps of a schedule of `sweeps` sweeps, in order, with a barrier between them.  Each lane
 // loads its half of a contact two steps ahead (record and accumulators), into the
 // registers of the one it has just solved: its accumulators were last written one step after the
 // last update, shift >= 4 steps before they are needed, so their writer has passed a barrier since.
-template <bool kGeneral, int kThreads>
-__device__ __forceinline__ void run_schedule(int levels, int shift, int stride, int sweeps,
+// `lanes`: of the block, those that take part, a multiple of 32.
+template <bool kGeneral>
+__device__ __forceinline__ void run_schedule(int lanes, int levels, int shift, int stride, int sweeps,
                                              float upper_bound, const int2* runs,
                                              const float4* rec, float2* accs, float4* vel,
                                              float4* ang, float4* vrel, int2* s_range) {
   const int steps = levels + (sweeps - 1) * shift;  // fits in int: checked by the host
-  constexpr int kTable = (kThreads - 2) / 2 * 2;    // steps per table, two more looked up
+  const int table = lanes - 2;                      // steps per table, even; two more looked up
   const int lane = threadIdx.x;  // this lane's half in a step's first round
   Rest rest;
   rest.v = rest.c = ar::mk3(0.f, 0.f, 0.f);
@@ -791,25 +794,25 @@ __device__ __forceinline__ void run_schedule(int levels, int shift, int stride, 
   auto solve = [&](Half& it, int2 r, int2 ahead) {
     if (__any_sync(0xffffffffu, it.h >= 0 || rest.h >= 0)) {
       solve_half<kGeneral>(it, accs, vel, ang, vrel, stride, upper_bound, rest);
-      for (int h0 = 2 * r.x + kThreads; h0 < 2 * r.y; h0 += kThreads) {
+      for (int h0 = 2 * r.x + lanes; h0 < 2 * r.y; h0 += lanes) {
         // contacts beyond one per lane pair
         load_half(rec, accs, h0 + lane < 2 * r.y ? h0 + lane : -1, it);
         solve_half<kGeneral>(it, accs, vel, ang, vrel, stride, upper_bound, rest);
       }
     }
     fetch(ahead, it);
-    __syncthreads();
+    lanes_barrier(lanes);
   };
   Half a, b;
-  for (int base = 1; base <= steps; base += kTable) {
+  for (int base = 1; base <= steps; base += table) {
     s_range[threadIdx.x] = step_range(base + (int)threadIdx.x, levels, sweeps, shift, runs);
-    __syncthreads();
+    lanes_barrier(lanes);
     if (base == 1) {
       fetch(s_range[0], a);
       fetch(s_range[1], b);
     }
-    const int count = min(kTable, steps - base + 1);
-    // two buffers in turn (a register move would wait for the loads in flight); kTable is even, so
+    const int count = min(table, steps - base + 1);
+    // two buffers in turn (a register move would wait for the loads in flight); `table` is even, so
     // every table starts with the same buffer
     for (int i = 0; i < count; i += 2) {
       solve(a, s_range[i], s_range[i + 2]);
@@ -830,17 +833,19 @@ __device__ __forceinline__ void run_schedule(int levels, int shift, int stride, 
 // and storing into the others' (a cluster barrier per step costs 0.7 us: 13 ms); copying the first
 // words to shared memory two steps ahead with cp.async (fewer stalls, a quarter more
 // instructions: 9.7 ms); three register buffers (spills: 28 ms).
-template <bool kShared, int kThreads>
-__global__ void __launch_bounds__(kThreads) sis_sweep_kernel(
+template <bool kShared>
+__global__ void __launch_bounds__(kSisThreads) sis_sweep_kernel(
     Bodies B, const int* __restrict__ hdr, int num_bodies, int schedule, int iterations,
     float upper_bound, const int2* __restrict__ run, const float4* __restrict__ rec,
     float2* __restrict__ accs, float4* __restrict__ vrel) {
   extern __shared__ float4 s_bodies[];  // (kShared) vel[num_bodies], ang[num_bodies]
-  __shared__ int2 s_range[kThreads];
+  __shared__ int2 s_range[kSisThreads];
+  __shared__ int s_widest;
   const int levels = hdr[kHdrLevels], shift = hdr[kHdrShift], count = hdr[kHdrCount];
   const int sweeps = sweeps_of(schedule, iterations, hdr);
-  if (sweeps == 0) return;
+  if (sweeps == 0 || levels == 0) return;
   float4 *vel = B.vel, *ang = B.ang;
+  if (threadIdx.x == 0) s_widest = 0;
   if (kShared) {
     vel = s_bodies;
     ang = s_bodies + num_bodies;
@@ -850,16 +855,24 @@ __global__ void __launch_bounds__(kThreads) sis_sweep_kernel(
     }
   }
   __syncthreads();
-  if (levels > 0) {
-    if (hdr[kHdrGeneral])
-      run_schedule<true, kThreads>(levels, shift, count, sweeps, upper_bound, run, rec, accs,
-                                   vel, ang, vrel, s_range);
-    else
-      run_schedule<false, kThreads>(levels, shift, count, sweeps, upper_bound, run, rec, accs,
-                                    vel, ang, vrel, s_range);
+  int widest = 0;
+  const int steps = levels + (sweeps - 1) * shift;
+  for (int step = 1 + (int)threadIdx.x; step <= steps; step += kSisThreads) {
+    const int2 r = step_range(step, levels, sweeps, shift, run);
+    widest = max(widest, r.y - r.x);
   }
-  if (kShared) {
-    for (int b = threadIdx.x; b < num_bodies; b += blockDim.x) {
+  atomicMax(&s_widest, widest);
+  __syncthreads();
+  const int lanes = min((2 * s_widest + 31) & ~31, kSisThreads);
+  if ((int)threadIdx.x >= lanes) return;
+  if (hdr[kHdrGeneral])
+    run_schedule<true>(lanes, levels, shift, count, sweeps, upper_bound, run, rec, accs, vel, ang,
+                       vrel, s_range);
+  else
+    run_schedule<false>(lanes, levels, shift, count, sweeps, upper_bound, run, rec, accs, vel, ang,
+                        vrel, s_range);
+  if (kShared) {  // (each step ends with a barrier)
+    for (int b = threadIdx.x; b < num_bodies; b += lanes) {
       B.vel[b] = vel[b];
       B.ang[b] = ang[b];
     }
@@ -999,20 +1012,17 @@ ar_status ar_sequential_impulse(ar_ctx* ctx, const ar_sim_params* params, const 
   sis_sizes_kernel<<<gg, 256, 0, st>>>(level, hdr, run);
   sis_layout_kernel<<<1, kLayoutThreads, 0, st>>>(hdr, run, order);
   sis_pack_kernel<<<gg, 256, 0, st>>>(C, B, geo, level, hdr, run, order, rec, accs);
-  // sweeps: the bodies' velocities in shared memory when they fit; more threads for scenes with
-  // many contacts per step
+  // sweeps: the bodies' velocities in shared memory when they fit
   const size_t body_smem = 32 * (size_t)num_bodies;
   const bool shared = body_smem <= kSisSmemMax;
   const size_t smem = shared ? body_smem : 0;
-  const bool many = num_bodies >= kSisManyBodies;
-  auto* sweep = !shared ? sis_sweep_kernel<false, kSisMany>
-                        : (many ? sis_sweep_kernel<true, kSisMany> : sis_sweep_kernel<true, kSisFew>);
+  auto* sweep = shared ? sis_sweep_kernel<true> : sis_sweep_kernel<false>;
   cudaFuncSetAttribute(sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // as many schedules as `capacity` contacts take; with fewer the last ones find no sweeps left
   const int fewest = (int)std::min((long long)iterations, slots / capacity);
   for (int i = 0; i * (long long)fewest < iterations; ++i) {
-    sweep<<<1, !shared || many ? kSisMany : kSisFew, smem, st>>>(
-        B, hdr, num_bodies, i, iterations, 100.f, run, rec, accs, vrel);
+    sweep<<<1, kSisThreads, smem, st>>>(B, hdr, num_bodies, i, iterations, 100.f, run, rec, accs,
+                                        vrel);
     sis_friction_kernel<<<gg, 256, 0, st>>>(C, geo, hdr, order, vrel, i, iterations, accs);
   }
   return arh::check_launch("ar_sequential_impulse");

@@ -412,18 +412,21 @@ struct Rest {
   int h = -1, sweep;
   float total;
   float3 v, c;  // the body's velocity before the update, and angular velocity x lever arm
+  bool slides = false;  // between two bodies
 };
 // The accumulated impulse, and the relative velocity for the friction as the reference sums it.
+template <bool kGeneral>
 __device__ __forceinline__ void store_rest(const Rest& r, float2* __restrict__ accs,
                                            float4* __restrict__ vrel, size_t stride) {
+  const bool first = r.h >= 0 && !(threadIdx.x & 1);
+  if (first) accs[r.h] = make_float2(r.total, __int_as_float(r.sweep + 1));
+  if (kGeneral && !__any_sync(0xffffffffu, r.slides)) return;
   auto pair = [&](float x) { return __shfl_xor_sync(0xffffffffu, x, 1); };
   const float3 v2 = ar::mk3(pair(r.v.x), pair(r.v.y), pair(r.v.z));
   const float3 c2 = ar::mk3(pair(r.c.x), pair(r.c.y), pair(r.c.z));
   const float3 slide = add3(add3(add3(mul3(-1.f, r.v), r.c), v2), c2);
-  if (r.h >= 0 && !(threadIdx.x & 1)) {
-    accs[r.h] = make_float2(r.total, __int_as_float(r.sweep + 1));
+  if (first && (!kGeneral || r.slides))
     vrel[(size_t)r.sweep * stride + (r.h >> 1)] = make_float4(slide.x, slide.y, slide.z, 0.f);
-  }
 }
 template <bool kGeneral>
 __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ accs, float4* vel,
@@ -443,7 +446,7 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
   const bool some = kGeneral && __any_sync(kAll, odd);
   const uint32_t other = some ? __shfl_xor_sync(kAll, tag, 1) : tag;
   const bool one = odd && (side ? tag : other) == kNoBody;
-  store_rest(rest, accs, vrel, stride);  // the previous update's
+  store_rest<kGeneral>(rest, accs, vrel, stride);  // the previous update's
   // the first lane's impulse against the second one's 1 / mc
   const float met = __shfl_xor_sync(kAll, it.acc.x, 1);
   const float acc = side ? met : it.acc.x;
@@ -499,7 +502,7 @@ __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ 
     vel[body] = make_float4(nv.x, nv.y, nv.z, 0.f);
     ang[body] = make_float4(nw.x, nw.y, nw.z, 0.f);
   }
-  rest = Rest{it.h, __float_as_int(it.acc.y), total, v, c};
+  rest = Rest{it.h, __float_as_int(it.acc.y), total, v, c, have && !one};
 }
 
 // Threads of the sweep block, two lanes per contact: a step's first 320 contacts are loaded ahead.
@@ -820,7 +823,7 @@ __device__ __forceinline__ void run_schedule(int lanes, int levels, int shift, i
       solve(b, s_range[i + 1], s_range[i + 3]);
     }
   }
-  store_rest(rest, accs, vrel, stride);
+  store_rest<kGeneral>(rest, accs, vrel, stride);
 }
 
 // The sweeps, in one block.  kShared: the bodies' velocities and angular velocities live in shared

@@ -135,8 +135,11 @@ __global__ void __launch_bounds__(256) build_few_kernel(Lcp lcp, int n, ar_lbvh:
   if (i < n - 1) ar_lbvh::karras_node(i, n, lcp, out);
 }
 
-// The tiles' barriers and the nodes that leave them cost a small tree more than the searches do:
-// 2,000 points 16.8 us against 15.8, 132,651 points 16.7 against 16.5.
+// The tiles' barriers and the nodes that leave them cost a small tree more than the searches do.
+// Where the two forms meet depends on the codes (kernels alone, searches against tiles: 30 spread
+// bits 100,000 points 10.4 / 11.5 us, 150,000 11.1 / 11.5, 200,000 11.6 / 11.9, 262,144 13.9 / 12.3;
+// 30 clustered bits 100,000 10.9 / 10.8, 150,000 12.1 / 11.2; 63 spread bits 100,000 11.9 / 12.1,
+// 131,072 12.8 / 11.9, 200,000 13.4 / 12.6): the line lies between.
 constexpr int kBuildTilesFrom = 1 << 17;
 template <class Lcp>
 void launch_build(const Lcp& lcp, int n, const ar_lbvh::TreeOut& out, cudaStream_t st) {
@@ -178,10 +181,10 @@ __global__ void __launch_bounds__(256) refit_kernel(int n, const int32_t* __rest
   if (i < n) ar_lbvh::refit_climb(i, n, left, right, parent, bounds, counters);
 }
 
-// From this many leaves on the tiles below pay for their second launch (both forms: 300,000 points
-// 47.7 us alone, 59.1 in tiles; 600,000: 69.6, 71.7; 1,000,003: 92.5, 89.1; 2,000,000: 151, 126;
-// with a climb that read both boxes and the links one after another: 57, 82, 110, 183).
-constexpr int kRefitTilesFrom = 1 << 20;
+// From this many leaves on the tiles below pay for their second launch (both forms: 400,000 points
+// 57.8 us alone, 65.2 in tiles; 600,000: 67.5, 70.7; 800,000: 77.6, 80.4; 900,000: 85.0, 83.0;
+// 1,000,003: 90.9, 87.6; 2,000,000: 150, 124).
+constexpr int kRefitTilesFrom = 7 << 17;
 // A block takes kRefitTile consecutive leaves and the internal nodes of the same numbers.  The
 // subtrees that lie within these are merged in shared memory, the second child to arrive at a node
 // merging both.  The largest of them are left to refit_open_kernel, which climbs the rest of the
@@ -266,7 +269,7 @@ __global__ void __launch_bounds__(kRefitTile) refit_tiles_kernel(int n, const in
   if (open_node) leave(n + k, at + (int)open_leaf);
 }
 
-// The climb from the subtrees that refit_kernel left over: a block collects those of kRefitScan
+// The climb from the subtrees that refit_tiles_kernel left over: a block collects those of kRefitScan
 // counters, so that its threads climb together.
 constexpr int kRefitScan = 4096;
 __global__ void __launch_bounds__(256) refit_open_kernel(int n, const int32_t* __restrict__ left,

@@ -249,8 +249,8 @@ __global__ void __launch_bounds__(256) scatter_kernel(
 // particles in 40 scenes: 227 -> 190 us against a walk that told the three cells apart and held
 // their partial sums) and by the latency of the 27 meta loads where they are not (2M pile: 58
 // us); loading 2, 4 or 8 candidates ahead changed nothing or lost occupancy.  Five blocks of 256
-// fit an SM with the scene table (a batch of one keeps its scene in the constant bank and more of
-// the rest in registers, where a fifth block spills and costs 2 %).
+// fit an SM with the scene table, at the price of 44 spilled bytes; a batch of one keeps its scene in
+// the constant bank, and there a fifth block costs 2 %.
 // The meta word of a cell that holds only this body, count bits cleared (an impossible word when
 // the body has no tag).
 __device__ __forceinline__ uint32_t own_meta(uint32_t epoch, uint32_t btag) {
@@ -703,7 +703,6 @@ struct __align__(64) WideNode {
 // its scene's root.
 template <bool kOne>
 struct StepTree {
-  static constexpr bool kBoxes = true;
   int32_t *left, *right, *parent, *roots;
   WideNode* nodes;
   const float4 *spos, *svel;
@@ -722,10 +721,10 @@ struct StepTree {
     const float4 p = __ldcg(spos + i);
     return record(ar::xyz(p), scene_at<kOne>(*one, table, scene_of(i)).r, i, __float_as_int(p.w));
   }
-  __device__ __forceinline__ void made(int id, int d, int dl, int dr, int first, int) const {
+  __device__ __forceinline__ void made(int id, int d, int dl, int dr, int first) const {
     if (d >= prefix && dl < prefix && dr < prefix) roots[scene_of(first)] = id;
   }
-  __device__ __forceinline__ void links(int id, int lc, int rc, int, int) const {
+  __device__ __forceinline__ void links(int id, int lc, int rc) const {
     left[id] = lc;
     right[id] = rc;
   }
@@ -786,7 +785,7 @@ __global__ void __launch_bounds__(ar_tree::kTile, 6) bvh_tree_kernel(
   __syncthreads();
   if (t < m && s.d[0][t] < out.prefix && s.d[0][t + 1] < out.prefix)
     out.roots[out.scene_of(k)] = -1;  // a scene of one particle
-  ar_tree::build_up(s, &box, m, n, lcp, out, work);
+  ar_tree::build_up(s, box, m, n, lcp, out, work);
 }
 
 // Half of a wide node in one 32-byte load.

@@ -1,4 +1,4 @@
-// Binary radix trees built a tile at a time, bottom up, with the boxes if wanted.
+// Binary radix trees built a tile at a time, bottom up, with their boxes.
 //
 // The tree over sorted keys follows from the prefix lengths d(s) = lcp(key s, key s + 1) of
 // neighbouring keys alone: the node whose children meet at split s covers the leaves between
@@ -11,7 +11,8 @@
 // descent through a table of range minima in shared memory; a node is closed when both lie
 // within the tile, borders included, and then its whole subtree does too.  What is left of a
 // tile are its largest closed subtrees, in order: they hang off the paths to its two borders, so
-// they are few (about a dozen for 256 leaves, and never more than 2 x 97).  The block that
+// they are few: the splits along a border's path have ever smaller prefixes, 97 lengths at most, so
+// there are no more than 2 x 97 + 1 subtrees (for 256 leaves usually about a dozen).  The block that
 // finishes last of kFan neighbouring ones takes their lists as its next tiles, subtrees in the
 // place of leaves, and so on up to the root, all within one launch.  Only that block reads what
 // the others wrote, behind one fence and counter per group, where a climb with an arrival counter
@@ -36,7 +37,7 @@ constexpr int kFan = 16;    // lists per group
 // listed nodes by number, a length and an arrival count per list (zero between launches).
 struct Scratch {
   int2* open;       // first and last leaf of a listed subtree; n entries
-  float4* pending;  // two per node; 2 n entries (unused without boxes)
+  float4* pending;  // two per node; 2 n entries
   int* length;      // lists_for(n)
   int* arrived;     // lists_for(n)
 };
@@ -68,7 +69,6 @@ struct Links {
   short top[kTile];                   // place of the largest closed subtree that starts here, -1
   int warp_sum[kTile / 32];
   int prefix[kFan + 1];               // of the group's list lengths
-  int total;
   bool last_of_group;
 };
 struct Boxes {
@@ -116,11 +116,11 @@ __device__ __forceinline__ void climb(Links& s, Boxes& box, int c) {
   }
 }
 
-// Finishes the closed nodes of a tile of m subtrees (first, last, d[0] up to d[0][m] and, with
-// boxes, the subtrees' records filled in, a barrier since) and leaves the largest closed subtrees
-// in `top`.  Every thread of the block calls it.
+// Finishes the closed nodes of a tile of m subtrees (first, last, d[0] up to d[0][m] and the
+// subtrees' records filled in, a barrier since) and leaves the largest closed subtrees in `top`.
+// Every thread of the block calls it.
 template <class Sink>
-__device__ __forceinline__ void close_nodes(Links& s, Boxes* box, int m, int n, const Sink& out) {
+__device__ __forceinline__ void close_nodes(Links& s, Boxes& box, int m, int n, const Sink& out) {
   const int t = threadIdx.x;
 #pragma unroll
   for (int k = 1; k < kLevels; ++k) {
@@ -147,37 +147,32 @@ __device__ __forceinline__ void close_nodes(Links& s, Boxes* box, int m, int n, 
     s.hi[num] = (short)hi;
     s.parent[lc] = s.parent[rc] = (short)num;
     s.made[num] = 1;
-    out.made(id, s.d[0][t], dl, dr, s.first[lo], s.last[hi - 1]);
+    out.made(id, s.d[0][t], dl, dr, s.first[lo]);
   }
   __syncthreads();
-  if constexpr (Sink::kBoxes) {
-    if (t < m) climb(s, *box, t);
-    __syncthreads();
-  }
+  if (t < m) climb(s, box, t);
+  __syncthreads();
   // links, by local number, and wide nodes by four threads each
   if (t < m && s.parent[t] >= 0) out.parent_of(s.id[t], s.id[kTile + s.parent[t]]);
   if (s.made[t]) {
     const int id = s.id[kTile + t];
-    out.links(id, s.id[s.child[0][t]], s.id[s.child[1][t]], s.first[s.lo[t]], s.last[s.hi[t] - 1]);
+    out.links(id, s.id[s.child[0][t]], s.id[s.child[1][t]]);
     if (s.parent[kTile + t] >= 0) out.parent_of(id, s.id[kTile + s.parent[kTile + t]]);
     else s.top[s.lo[t]] = (short)(kTile + t);
   }
   if (t < m && s.parent[t] < 0) s.top[t] = (short)t;
-  if constexpr (Sink::kBoxes) {
-    for (int i = t; i < 4 * kTile; i += kTile) {
-      const int node = i >> 2;
-      if (!s.made[node]) continue;
-      const int c = s.child[(i >> 1) & 1][node];
-      out.wide(s.id[kTile + node] - n, i & 3, i & 1 ? box->b[c] : box->a[c]);
-    }
+  for (int i = t; i < 4 * kTile; i += kTile) {
+    const int node = i >> 2;
+    if (!s.made[node]) continue;
+    const int c = s.child[(i >> 1) & 1][node];
+    out.wide(s.id[kTile + node] - n, i & 3, i & 1 ? box.b[c] : box.a[c]);
   }
   __syncthreads();
 }
 
 // Appends the tile's largest closed subtrees, in order, to the list at `to`, which holds `have`
 // already; returns its new length.
-template <class Sink>
-__device__ __forceinline__ int list_open(Links& s, const Boxes* box, int m, int n, int2* to,
+__device__ __forceinline__ int list_open(Links& s, const Boxes& box, int m, int n, int2* to,
                                          int have, const Scratch& w) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int c = t < m ? s.top[t] : -1;
@@ -192,10 +187,10 @@ __device__ __forceinline__ int list_open(Links& s, const Boxes* box, int m, int 
   if (c >= 0) {
     const int last = c < kTile ? s.last[t] : s.last[s.hi[c - kTile] - 1];
     __stcg(to + at + __popc(some & ((1u << lane) - 1)), make_int2(s.first[t], last));
-    if (Sink::kBoxes && c >= kTile) {
+    if (c >= kTile) {
       float4* p = w.pending + 2 * (size_t)(s.id[c] - n);
-      __stcg(p, box->a[c]);
-      __stcg(p + 1, box->b[c]);
+      __stcg(p, box.a[c]);
+      __stcg(p + 1, box.b[c]);
     }
   }
   __syncthreads();
@@ -212,13 +207,13 @@ __device__ __forceinline__ void reset_links(Links& s) {
 // The tree above a block's tile.  The tile's subtrees are in s (and box), filled in by the caller
 // up to d[0]; `sink.leaf(i)` is the record of leaf i, readable once its block has arrived.
 template <class Lcp, class Sink>
-__device__ __forceinline__ void build_up(Links& s, Boxes* box, int m, int n, const Lcp& lcp,
+__device__ __forceinline__ void build_up(Links& s, Boxes& box, int m, int n, const Lcp& lcp,
                                          const Sink& sink, const Scratch& w) {
   const int t = threadIdx.x;
   close_nodes(s, box, m, n, sink);
   int unit = blockIdx.x, units = gridDim.x, lists = 0;  // `lists`: of the levels below
   long span = kTile;                                    // leaves per list
-  int length = list_open<Sink>(s, box, m, n, w.open + (size_t)unit * span, 0, w);
+  int length = list_open(s, box, m, n, w.open + (size_t)unit * span, 0, w);
   while (units > 1) {
     const int group = unit / kFan, count = min(kFan, units - group * kFan);
     // the block's boxes, lists and leaves are ordered before its arrival by the barrier and the
@@ -250,7 +245,7 @@ __device__ __forceinline__ void build_up(Links& s, Boxes* box, int m, int n, con
     int have = s.prefix[kFan];
     bool joined = false;  // the lists have become one
     // once through the group's subtrees, a tile at a time; at the top until one is left (a tile
-    // of 256 leaves at most 195, so a few passes; the bound only guards against unsorted keys)
+    // leaves at most 195 of 256, so a few passes; the bound only guards against unsorted keys)
     int pass = 0;
     do {
       int kept = 0;
@@ -275,21 +270,19 @@ __device__ __forceinline__ void build_up(Links& s, Boxes* box, int m, int n, con
           if (t == c - 1) s.d[0][c] = (signed char)dr;
           const int number = dr > dl ? e.y : e.x;
           s.id[t] = e.x == e.y ? e.x : n + number;
-          if constexpr (Sink::kBoxes) {
-            Box2 r;
-            if (e.x == e.y) {
-              r = sink.leaf(e.x);
-            } else {
-              const float4* p = w.pending + 2 * (size_t)number;
-              r = Box2{__ldcg(p), __ldcg(p + 1)};
-            }
-            box->a[t] = r.a;
-            box->b[t] = r.b;
+          Box2 r;
+          if (e.x == e.y) {
+            r = sink.leaf(e.x);
+          } else {
+            const float4* p = w.pending + 2 * (size_t)number;
+            r = Box2{__ldcg(p), __ldcg(p + 1)};
           }
+          box.a[t] = r.a;
+          box.b[t] = r.b;
         }
         __syncthreads();  // the tile is read before its place in the list is written over
         close_nodes(s, box, c, n, sink);
-        kept = list_open<Sink>(s, box, c, n, w.open + at, kept, w);
+        kept = list_open(s, box, c, n, w.open + at, kept, w);
       }
       have = kept;
       joined = true;

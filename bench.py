@@ -58,12 +58,23 @@ def sort_passes(bits: int) -> int:
     return (bits + 8) // 9 if bits > 0 else 0
 
 
+def resort_tiles(n: int) -> int:
+    """Tiles of the re-sort (csrc/ar_resort.cuh: tile_for)."""
+    tile = 512 if n < 1 << 18 else 2048
+    return (n + tile - 1) // tile
+
+
+def sort64_tiles(n: int) -> int:
+    """Tiles of a digit pass over 64-bit keys (csrc/ar_sort.cu: tile_items)."""
+    tile = 512 * 8 if n >= 1 << 19 else 256 * 8
+    return (n + tile - 1) // tile
+
+
 def stage_bytes(n: int, nb: int, passes: int, occupied_cells: int,
                 cells: int = 0) -> dict[str, float]:
     """Algorithmic bytes of one grid step that re-sorts from the previous order (every step
     but the first after a change of the member list).  The movers' own bytes (about 1 % of the
     particles, 8-16 bytes each per kernel) are left out."""
-    tiles = (n + 2047) // 2048
     return {
         # re-sort counters and bucket counts; one 255th of the 8-byte cell table
         "clear": 4 * (4 + 2 * 4096) + 8 * cells // 255,
@@ -71,7 +82,7 @@ def stage_bytes(n: int, nb: int, passes: int, occupied_cells: int,
         "keys": n * (16 + 4) + nb * 32,
         # movers: previous keys + indices in, new key gathered, mover bits out; placement:
         # previous keys + indices and mover bits in, keys + indices out; tile counts/headers
-        "sort": n * (8 + 4 + 0.125) + n * (8 + 0.125 + 8) + tiles * 40,
+        "sort": n * (8 + 4 + 0.125) + n * (8 + 0.125 + 8) + resort_tiles(n) * 40,
         # sorted key + index and rel in, sorted position + velocity and the order kept for the
         # next step out; body state per body; one 8-byte cell entry per occupied cell
         "scatter": n * (8 + 16 + 32 + 8) + nb * BODY_STATE + occupied_cells * 8,
@@ -89,7 +100,6 @@ def stage_bytes_bvh(n: int, nb: int, passes: int, key_bits: int = 64) -> dict[st
     """The same accounting for the BVH broad phase (64-byte wide nodes).  Keys of up to 32 bits
     (up to four scenes) are re-sorted from the previous step's order after the first step
     (movers' own bytes left out); wider keys are radix-sorted as 64-bit keys."""
-    tiles = (n + 8191) // 8192
     k32 = key_bits <= 32
     return {
         "clear": 4 * (4 + 2 * 4096) if k32 else 0,  # the re-sort's counters
@@ -98,8 +108,8 @@ def stage_bytes_bvh(n: int, nb: int, passes: int, key_bits: int = 64) -> dict[st
         # re-sort: previous keys + indices in, new key gathered, mover bits; placement: previous
         # keys + indices and bits in, keys + indices out.  Radix: histogram pass reads the keys;
         # first pass reads keys, every pass writes key + index, later passes read both
-        "sort": (n * (8 + 4 + 0.125) + n * (8 + 0.125 + 8) + (n // 2048) * 40) if k32 else
-                n * 8 + n * (8 + 12) + (passes - 1) * n * 24 + passes * 4 * 512 * tiles,
+        "sort": (n * (8 + 4 + 0.125) + n * (8 + 0.125 + 8) + resort_tiles(n) * 40) if k32 else
+                n * 8 + n * (8 + 12) + (passes - 1) * n * 24 + passes * 4 * 512 * sort64_tiles(n),
         # keys, index and rel in, body state per body; sorted pos + vel out (and the order kept,
         # 32-bit keys); links and the wide node out
         "tree": n * ((4 if k32 else 8) + 4 + 16 + 32) + (n * 8 if k32 else 0) +

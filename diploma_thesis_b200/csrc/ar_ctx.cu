@@ -96,7 +96,8 @@ void* scratch(ar_ctx* ctx, size_t need, size_t want, cudaStream_t st) {
     return p ? p : scratch(ctx, need);
   }
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  const bool may_grow = !ctx->reserved && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+  const bool may_grow = !ctx->reserved && want < ctx->denied &&
+                        cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
                         capture == cudaStreamCaptureStatusNone;
   if (may_grow) {
     void* more = nullptr;
@@ -111,6 +112,7 @@ void* scratch(ar_ctx* ctx, size_t need, size_t want, cudaStream_t st) {
       ctx->reserved = false;
       return more;
     }
+    ctx->denied = want;
   }
   cudaGetLastError();
   return ctx->scratch;

@@ -104,6 +104,7 @@ struct ar_ctx {
   void* scratch = nullptr;     // grow-only arena
   size_t scratch_bytes = 0;
   bool reserved = false;       // the arena's size is what ar_ctx_reserve made it
+  size_t denied = SIZE_MAX;    // wanted, not needed, and not to be had: not asked for again
   int num_sms = 148;
 };
 

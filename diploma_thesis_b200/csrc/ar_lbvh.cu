@@ -137,9 +137,9 @@ __global__ void __launch_bounds__(256) build_few_kernel(Lcp lcp, int n, ar_lbvh:
 
 // The tiles' barriers and the nodes that leave them cost a small tree more than the searches do.
 // Where the two forms meet depends on the codes (kernels alone, searches against tiles: 30 spread
-// bits 100,000 points 10.4 / 11.5 us, 150,000 11.1 / 11.5, 200,000 11.6 / 11.9, 262,144 13.9 / 12.3;
-// 30 clustered bits 100,000 10.9 / 10.8, 150,000 12.1 / 11.2; 63 spread bits 100,000 11.9 / 12.1,
-// 131,072 12.8 / 11.9, 200,000 13.4 / 12.6): the line lies between.
+// bits 100,000 points 10.4 / 11.5 us, 150,000 11.1 / 11.5, 200,000 11.6 / 11.9, 262,144 13.9 /
+// 12.3; 30 clustered bits 100,000 10.9 / 10.8, 150,000 12.1 / 11.2; 63 spread bits 100,000 11.9 /
+// 12.1, 131,072 12.8 / 11.9, 200,000 13.4 / 12.6): the line lies between.
 constexpr int kBuildTilesFrom = 1 << 17;
 template <class Lcp>
 void launch_build(const Lcp& lcp, int n, const ar_lbvh::TreeOut& out, cudaStream_t st) {

@@ -140,7 +140,8 @@ __device__ __forceinline__ void refit_climb(int from, int n, const int32_t* __re
                                             const int32_t* __restrict__ right,
                                             const int32_t* __restrict__ parent, float4* bounds,
                                             int* counters) {
-  auto inner = [&](int node) { return node >= n && node < 2 * n - 1; };  // else malformed, or no node
+  // else the link is malformed, or there is no node
+  auto inner = [&](int node) { return node >= n && node < 2 * n - 1; };
   int child = from, node = __ldg(parent + from);
   Box6 own = box6(__ldcg(bounds + 2 * (size_t)from), __ldcg(bounds + 2 * (size_t)from + 1));
   if (!inner(node)) return;
@@ -194,8 +195,8 @@ __device__ __forceinline__ bool overlap(const Box& a, const Box& b) {
 // over 32-bit keys rarely needs more.  Older ones are dropped, and found again once the stack is
 // empty by climbing the parent links from the subtree just finished, so that no depth is too
 // great.  Climbing after every subtree instead reads each node's links and boxes a second time on
-// the way up (132,651 packed particles: 341 -> 175 us).  A valid tree is walked in fewer than 4 (2n - 1) moves; the bound only
-// guards against a malformed tree.
+// the way up (132,651 packed particles: 341 -> 175 us).  A valid tree is walked in fewer than
+// 4 (2n - 1) moves; the bound only guards against a malformed tree.
 constexpr int kStack = 32;  // a power of two
 template <class Accept, class Visit>
 __device__ __forceinline__ void walk(int root, int n, const int32_t* __restrict__ left,

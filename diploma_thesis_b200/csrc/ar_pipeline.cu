@@ -742,9 +742,10 @@ struct StepTree {
 // climbed with a device-scope arrival per node, and a root search (2M pile: 275 -> 184 us; 12
 // scenes, 290k particles, 64-bit keys: 91 -> 62 us).  Bound by latency and issue: 1,200 warp
 // instructions per 32 leaves, half of the issue slots used, then about 45 us of the last groups'
-// levels with most SMs idle.  Tiles of 128 (217 us) leave twice the subtrees to the levels above;
-// groups of 8 or 32 lists add a level or a tile to each (197, 236 us); finishing the nodes in
-// block-wide rounds instead of the climb executed 30 % more instructions.
+// levels with most SMs idle (six blocks per SM, 20 to 44 bytes of each thread spilled).  Tiles of
+// 128 (217 us) leave twice the subtrees to the levels above; groups of 8 or 32 lists add a level or
+// a tile to each (197, 236 us); finishing the nodes in block-wide rounds instead of the climb
+// executed 30 % more instructions.
 template <class Lcp, bool kOne>
 __global__ void __launch_bounds__(ar_tree::kTile, 6) bvh_tree_kernel(
     const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table,
@@ -1482,8 +1483,8 @@ ar_status enqueue_step(ar_batch* B, cudaStream_t st, cudaEvent_t* ev = nullptr) 
     if (s != AR_OK) return s;
   }
   mark(3);
-  AR_LAUNCH_ONE(scatter_kernel, dim3(arh::grid_for(nt, 256)), dim3(256), B->d_table, B->d_pscene, nt, B->skeys,
-      B->svals, B->cells, B->spos, B->svel, B->pkeys, B->pvals, B->d_step);
+  AR_LAUNCH_ONE(scatter_kernel, dim3(arh::grid_for(nt, 256)), dim3(256), B->d_table, B->d_pscene,
+      nt, B->skeys, B->svals, B->cells, B->spos, B->svel, B->pkeys, B->pvals, B->d_step);
   mark(4);
   if (nt <= ctx->num_sms * kFewPerSm) {
     const int per_warp = per_warp_for(ctx, nt, kFewWarps);

@@ -377,7 +377,7 @@ struct Half {
 };
 // Loads at this point of the program: the compiler would move plain loads down to their uses, a
 // step later, to save registers.  Through L1, which holds a small list: its steps are shorter than
-// two steps' way to L2 (200 bodies in a chain, 300 sweeps: 1.24 -> 1.14 ms, 27 cubes of 8: 0.75 ->
+// two steps' way to L2 (200 bodies in a chain, 300 sweeps: 1.24 -> 1.14 ms, 27 cubes of 8 0.75 ->
 // 0.63; large lists the same).
 __device__ __forceinline__ float4 load_now(const float4* p) {
   float4 v;
@@ -399,13 +399,6 @@ __device__ __forceinline__ void load_half(const float4* rec, const float2* accs,
   it.acc = load_now(accs + h);
 }
 
-// One contact's update, the velocity-dependent part of the reference's loop body, by the two
-// lanes that hold its halves (every lane of the warp calls it).  Each lane takes its body's share
-// of the relative velocity, both compute the impulse, and each updates its body.  Friction between
-// two bodies is accumulated but never applied (as in the reference), so only the relative velocity
-// it needs is kept, in `vrel`, for sis_friction_kernel.  Lanes without a contact compute along on
-// what their registers hold, so they must not decide on a warp's plain division.  kGeneral: some
-// contact of the list is odd (else the compiler leaves the tests for it out).
 // What an update leaves to be stored: no other update waits for it, so it is done in the next
 // step, between that step's dependent operations.
 struct Rest {
@@ -428,6 +421,13 @@ __device__ __forceinline__ void store_rest(const Rest& r, float2* __restrict__ a
   if (first && (!kGeneral || r.slides))
     vrel[(size_t)r.sweep * stride + (r.h >> 1)] = make_float4(slide.x, slide.y, slide.z, 0.f);
 }
+// One contact's update, the velocity-dependent part of the reference's loop body, by the two
+// lanes that hold its halves (every lane of the warp calls it).  Each lane takes its body's share
+// of the relative velocity, both compute the impulse, and each updates its body.  Friction between
+// two bodies is accumulated but never applied (as in the reference), so only the relative velocity
+// it needs is kept, in `vrel`, for sis_friction_kernel.  Lanes without a contact compute along on
+// what their registers hold, so they must not decide on a warp's plain division.  kGeneral: some
+// contact of the list is odd (else the compiler leaves the tests for it out).
 template <bool kGeneral>
 __device__ __forceinline__ void solve_half(const Half& it, float2* __restrict__ accs, float4* vel,
                                            float4* ang, float4* __restrict__ vrel, size_t stride,
@@ -514,9 +514,11 @@ constexpr size_t kSisSmemMax = 220 * 1024;   // the sweep block's dynamic shared
 constexpr size_t kWalkSmemMax = 200 * 1024;  // the walk's (its static 16 KB stay below 227 KB)
 // Relative velocities kept at most, 16 bytes each (one per contact and sweep of a schedule).
 constexpr long long kMaxSlots = 1l << 25;
-// The schedule's header in scratch memory: levels, shift, contact count, whether some contact needs
-// the general update, and sweeps per schedule.
-enum { kHdrLevels = 0, kHdrShift = 1, kHdrCount = 2, kHdrGeneral = 3, kHdrSweeps = 4, kHdrWords = 8 };
+// The schedule's header in scratch memory: levels, shift, contact count, whether some contact is odd,
+// and sweeps per schedule.
+enum {
+  kHdrLevels = 0, kHdrShift = 1, kHdrCount = 2, kHdrGeneral = 3, kHdrSweeps = 4, kHdrWords = 8
+};
 
 // Schedule.  Each contact gets a level: 1 + the highest level among earlier contacts on either
 // of its bodies.  Sweep s solves level b at step b + s * shift of one schedule, where shift
@@ -782,8 +784,8 @@ __device__ __forceinline__ void lanes_barrier(int lanes) {
 // last update, shift >= 4 steps before they are needed, so their writer has passed a barrier since.
 // `lanes`: of the block, those that take part, a multiple of 32.
 template <bool kGeneral>
-__device__ __forceinline__ void run_schedule(int lanes, int levels, int shift, int stride, int sweeps,
-                                             float upper_bound, const int2* runs,
+__device__ __forceinline__ void run_schedule(int lanes, int levels, int shift, int stride,
+                                             int sweeps, float upper_bound, const int2* runs,
                                              const float4* rec, float2* accs, float4* vel,
                                              float4* ang, float4* vrel, int2* s_range) {
   const int steps = levels + (sweeps - 1) * shift;  // fits in int: checked by the host
@@ -828,14 +830,14 @@ __device__ __forceinline__ void run_schedule(int lanes, int levels, int shift, i
 
 // The sweeps, in one block.  kShared: the bodies' velocities and angular velocities live in shared
 // memory.
-// Bound by the serial chain of steps and by issue on one SM: 7,966 steps of up to 282 contacts on
-// 4,096 packed cubes, 0.93 us each, of which a contact's dependent operations, a barrier and 190
-// instructions per warp.  13.7 -> 7.4 ms against a lane per contact with divisions (510
-// instructions), its friction and its accumulators before the barrier, and loads one step ahead
-// that the step did not cover.  Tried: a cluster of two or four blocks, each with all velocities
-// and storing into the others' (a cluster barrier per step costs 0.7 us: 13 ms); copying the first
-// words to shared memory two steps ahead with cp.async (fewer stalls, a quarter more
-// instructions: 9.7 ms); three register buffers (spills: 28 ms).
+// Bound by the serial chain of steps and by issue on one SM: 8,052 steps of up to 282 contacts on
+// 4,096 packed cubes, 0.9 us each: a contact's dependent operations, a barrier and 160
+// instructions per warp (40 % of the SM's issue slots).  13.7 -> 7.3 ms against a lane per contact
+// with divisions (510 instructions), its friction and its accumulators before the barrier, and
+// loads one step ahead that the step did not cover.  Tried: a cluster of two or four blocks, each
+// with all velocities and storing into the others' (a cluster barrier per step costs 0.7 us: 13
+// ms); copying the first words to shared memory two steps ahead with cp.async (fewer stalls, a
+// quarter more instructions: 9.7 ms); three register buffers (spills: 28 ms).
 template <bool kShared>
 __global__ void __launch_bounds__(kSisThreads) sis_sweep_kernel(
     Bodies B, const int* __restrict__ hdr, int num_bodies, int schedule, int iterations,

@@ -214,7 +214,9 @@ AR_API ar_status ar_lbvh_refit(ar_ctx* ctx, int n, const int32_t* left, const in
  * nodes to return to and finds older ones through the parent links, so no per-thread stack
  * limits the tree depth; `parent` may be NULL (the
  * reference's wrapper signature has none), in which case the links are derived from
- * left/right first.  Contacts are visited in the reference's order. */
+ * left/right first.  Contacts are visited in the reference's order.  Here and in the other
+ * traversals is_leaf must be given, as in the reference's signatures, but is not read: leaves are
+ * the nodes below n. */
 AR_API ar_status ar_collide_bvh_dem(ar_ctx* ctx, const ar_sim_params* params,
                                     const int32_t* rb_idx, const float* rel4,
                                     const float* vel4, const uint8_t* is_leaf,
@@ -646,8 +648,8 @@ AR_API ar_status ar_scene_destroy_async(ar_scene* scene, ar_stream_t stream);
  * is sorted once.  num_points = 0 detaches the cloud.  Synchronises the device (steps in
  * flight may read the old cloud).  A cloud of no more points than the scene's largest so far
  * is sorted into the buffers the scene has; attaching the first or a larger one, or detaching,
- * makes every batch holding the scene rebuild its table before its next step.  A clone (ar_scene_clone_async) starts without a cloud.  BVH scenes:
- * AR_ERR_INVALID_ARG. */
+ * makes every batch holding the scene rebuild its table before its next step.  A clone
+ * (ar_scene_clone_async) starts without a cloud.  BVH scenes: AR_ERR_INVALID_ARG. */
 AR_API ar_status ar_scene_set_static_cloud(ar_ctx* ctx, ar_scene* scene, const float* cloud_pos4,
                                            const float* cloud_norm4, int num_points,
                                            ar_stream_t stream);

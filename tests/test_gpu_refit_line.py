@@ -1,4 +1,4 @@
-"""ar_lbvh_refit on both sides of the size from which subtrees are merged in tiles (7 x 2^17 leaves)."""
+"""ar_lbvh_refit on both sides of the size from which subtrees merge in tiles (7 x 2^17 leaves)."""
 import pytest
 
 from test_gpu_refit_tiles import test_refit_forms as refit_forms

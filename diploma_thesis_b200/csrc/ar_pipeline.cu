@@ -498,7 +498,9 @@ __global__ void __launch_bounds__(256) collide_few_kernel(
 // per_warp: a scene with few particles spreads them over as many warps as the chip holds, one
 // with many keeps the lanes busy in the first pass, where most particles find no points.
 constexpr float kLaneWalk = 1.5f;  // rounds that a point of the longest lane is worth
-template <bool kOne>
+// kLanes: with the lanes' walk, which needs two particles per warp to be the shorter one; the kernel
+// without it is 1 us faster (a 640 x 480 cloud's step of 3,200 particles: 48.7 -> 47.7 us).
+template <bool kOne, bool kLanes>
 __global__ void __launch_bounds__(128) cloud_collide_kernel(
     const __grid_constant__ SceneDev one, const SceneDev* __restrict__ table, int nt, int per_warp,
     const uint32_t* __restrict__ skeys, const uint32_t* __restrict__ svals,
@@ -521,13 +523,12 @@ __global__ void __launch_bounds__(128) cloud_collide_kernel(
       for (int r = 0; r < 27; ++r) {
         const uint2 c = __ldg(cc + near_cell(S, key - S.cell_base, r));
         todo |= (c.x < c.y ? 1u : 0u) << r;
-        points += c.y - c.x;
+        if (kLanes) points += c.y - c.x;
       }
     }
   }
-  const uint32_t rounds = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(todo) + points / 32);
-  if (rounds == 0) return;
-  if (kLaneWalk * __reduce_max_sync(0xffffffffu, points) <= rounds) {
+  if (kLanes && kLaneWalk * __reduce_max_sync(0xffffffffu, points) <=
+                    __reduce_add_sync(0xffffffffu, (uint32_t)__popc(todo) + points / 32)) {
     const SceneDev& S = scene_at<kOne>(one, table, kOne ? 0 : __float_as_int(v4.w));
     const float3 pos = ar::xyz(p4), vel = ar::xyz(v4);
     const float thr = 2.0f * S.r;
@@ -1497,7 +1498,10 @@ ar_status enqueue_step(ar_batch* B, cudaStream_t st, cudaEvent_t* ev = nullptr) 
   }
   if (B->has_cloud) {
     const int per_warp = per_warp_for(ctx, nt, kCloudWarps);
-    AR_LAUNCH_ONE(cloud_collide_kernel, dim3(arh::grid_for(nt, 4 * per_warp)), dim3(128),
+    auto* kernel = per_warp > 1
+        ? (one ? cloud_collide_kernel<true, true> : cloud_collide_kernel<false, true>)
+        : (one ? cloud_collide_kernel<true, false> : cloud_collide_kernel<false, false>);
+    arh::launch_pdl(kernel, dim3(arh::grid_for(nt, 4 * per_warp)), dim3(128), 0, st, B->one,
         B->d_table, nt, per_warp, B->skeys, B->svals, B->spos, B->svel, B->pforce);
   }
   mark(5);

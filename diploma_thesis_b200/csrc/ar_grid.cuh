@@ -31,15 +31,16 @@ struct Grid {
 };
 
 // Calls visit(first, end) for every occupied cell among the 27 around `c`, in z, y, x order, with
-// its range of sorted slots.  The cell starts of a row are loaded one row ahead; empty cells are
+// its range of sorted slots, and row_done() after every row of three.  The cell starts of a row are loaded one row ahead; empty cells are
 // passed over (a float sum that starts at +0 is never -0, so the +0 that an empty cell would add
 // changes nothing).  All lanes of a warp look at the same neighbour at a time, so that their
 // loads, like their cells, lie side by side: letting each lane jump to its next occupied cell
 // scattered the loads and was slower.
-template <class Visit>
+template <class Visit, class RowDone>
 __device__ __forceinline__ void for_occupied(const Grid& g, int3 c,
                                              const uint32_t* __restrict__ cell_start,
-                                             const uint32_t* __restrict__ cell_end, Visit visit) {
+                                             const uint32_t* __restrict__ cell_end, Visit visit,
+                                             RowDone row_done) {
   uint32_t x[3], start[3], next[3];
 #pragma unroll
   for (int i = 0; i < 3; ++i) x[i] = (uint32_t)(c.x + i - 1) & (g.gx - 1);
@@ -68,7 +69,14 @@ __device__ __forceinline__ void for_occupied(const Grid& g, int3 c,
 #pragma unroll
     for (int i = 0; i < 3; ++i)
       if (start[i] != ar::kEmpty) visit(start[i], end[i]);
+    row_done();
   }
+}
+template <class Visit>
+__device__ __forceinline__ void for_occupied(const Grid& g, int3 c,
+                                             const uint32_t* __restrict__ cell_start,
+                                             const uint32_t* __restrict__ cell_end, Visit visit) {
+  for_occupied(g, c, cell_start, cell_end, visit, [] {});
 }
 
 }  // namespace ar_grid
